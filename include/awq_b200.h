@@ -379,9 +379,8 @@ int awq_b200_gemm_decode_f8(const void *A, int a_format, const int32_t *qweight,
  * xrt.py:204-218. */
 int awq_b200_gemm_check(awq_stream_t stream);
 
-/* Choose the prefill kernel: 0 = automatic, 1 = generic CUDA-core kernel, 2 = tcgen05 kernel with the
- * dequantised weights as a shared-memory tile, 3 = tcgen05 kernel with the dequantised weights in tensor
- * memory (2 and 3: AWQ_ERR_UNSUPPORTED where they cannot run; automatic takes 3 from 1024 rows on). */
+/* Choose the prefill kernel: 0 = automatic, 1 = generic CUDA-core kernel, 2 or 3 = the tcgen05 kernel
+ * (AWQ_ERR_UNSUPPORTED where it cannot run; automatic takes it wherever it can). */
 int awq_b200_set_gemm_kernel(int mode);
 
 /* ---- bf16 sibling path (un-quantised weights) ----------------------------------------------

@@ -337,14 +337,11 @@ extern "C" int awq_b200_gemm_bf16(const uint16_t *A, const int32_t *qweight, con
     AWQ_REQUIRE(A && qweight && qzeros && scales && C, "gemm: null pointer");
     AWQ_REQUIRE(aligned16(A) && aligned16(scales), "gemm: A and scales must be 16-byte aligned");
     const int mode = g_gemm_mode.load();
-    const bool tc_ok = gemm_tc_supported(M, K, N, group_size) && aligned16(qweight) && aligned16(qzeros) && aligned16(C);
-    if (mode == 2 && !tc_ok)
+    const bool tc_ok = gemm_pair_supported(M, K, N, group_size) && aligned16(qweight) && aligned16(qzeros) && aligned16(C);
+    if (mode >= 2 && !tc_ok)
         return set_error(AWQ_ERR_UNSUPPORTED, "gemm: tensor-core kernel does not cover M=%d K=%d N=%d gs=%d", M, K, N,
                          group_size);
-    // automatic: from 1024 rows on the kernel that keeps the dequantised weights in tensor memory measured faster
-    // (194 against 212 us on 2048 x 4096 x 14336), below that the tile with the weights in shared memory
-    if ((mode == 3 || (mode == 0 && M >= 1024)) && tc_ok) return launch_gemm_tm(A, qweight, qzeros, scales, C, M, K, N, as_stream(stream));
-    if (mode != 1 && tc_ok) return launch_gemm_tc(A, qweight, qzeros, scales, C, M, K, N, group_size, as_stream(stream));
+    if (mode != 1 && tc_ok) return launch_gemm_pair(A, qweight, qzeros, scales, C, M, K, N, as_stream(stream));
     return launch_gemm_generic(A, qweight, qzeros, scales, C, M, K, N, group_size, as_stream(stream));
 }
 
@@ -357,20 +354,18 @@ extern "C" int awq_b200_gemm_fused_bf16(const uint16_t *A, const int32_t *qweigh
     AWQ_REQUIRE(A && qweight && qzeros && scales && C, "gemm_fused: null pointer");
     AWQ_REQUIRE(aligned16(A) && aligned16(scales) && aligned16(qweight) && aligned16(qzeros) && aligned16(C) &&
                     aligned16(residual), "gemm_fused: pointers must be 16-byte aligned");
-    if (!gemm_tc_supported(M, K, N, group_size) || g_gemm_mode.load() == 1)
+    if (!gemm_pair_supported(M, K, N, group_size) || g_gemm_mode.load() == 1)
         return set_error(AWQ_ERR_UNSUPPORTED, "gemm_fused: needs the tensor-core kernel (group 128, K %% 128 == 0, N %% 32 == 0; "
                          "M=%d K=%d N=%d gs=%d)", M, K, N, group_size);
     const int epi = swiglu ? GEMM_EPI_SWIGLU : (residual ? GEMM_EPI_RESIDUAL : GEMM_EPI_BF16);
-    if (g_gemm_mode.load() == 3 || (g_gemm_mode.load() == 0 && M >= 1024)) return launch_gemm_tm(A, qweight, qzeros, scales, C, M, K, N, as_stream(stream), epi, residual);
-    return launch_gemm_tc(A, qweight, qzeros, scales, C, M, K, N, group_size, as_stream(stream), epi, residual);
+    return launch_gemm_pair(A, qweight, qzeros, scales, C, M, K, N, as_stream(stream), epi, residual);
 }
 
 extern "C" int awq_b200_gemm_check(awq_stream_t stream) {
-    const int rc = gemm_tc_check(as_stream(stream));
+    const int rc = gemm_pair_check(as_stream(stream));
     const int rc2 = gemm_decode_check(as_stream(stream));
-    const int rc3 = gemm_tm_check(as_stream(stream));
-    const int rc4 = gemm_decode_f8_check(as_stream(stream));
-    return rc ? rc : (rc2 ? rc2 : (rc3 ? rc3 : rc4));
+    const int rc3 = gemm_decode_f8_check(as_stream(stream));
+    return rc ? rc : (rc2 ? rc2 : rc3);
 }
 
 extern "C" size_t awq_b200_gemm_decode_workspace_bytes(int M, int N) { return gemm_decode_workspace_bytes(M, N); }

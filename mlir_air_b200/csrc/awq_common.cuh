@@ -141,20 +141,16 @@ size_t gemv_streamk_workspace_clear_bytes(int N);
 int launch_gemm_generic(const uint16_t *A, const int32_t *qweight, const int32_t *qzeros,
                         const uint16_t *scales, uint16_t *C, int M, int K, int N, int group_size,
                         cudaStream_t stream);
-bool gemm_tc_supported(int M, int K, int N, int group_size);
 // Epilogues of the tensor-core GEMM: C bf16 [M, N] = bf16(sum (+ residual)), or SwiGLU over interleaved
 // gate/up column pairs into C bf16 [M, N / 2].
 enum GemmEpilogue : int { GEMM_EPI_BF16 = 0, GEMM_EPI_RESIDUAL = 1, GEMM_EPI_SWIGLU = 2, GEMM_EPI_F32 = 3 };  // F32: the f32 sums as they are (batched-decode GEMM only)
-int launch_gemm_tc(const uint16_t *A, const int32_t *qweight, const int32_t *qzeros,
-                   const uint16_t *scales, uint16_t *C, int M, int K, int N, int group_size,
-                   cudaStream_t stream, int epilogue = GEMM_EPI_BF16, const uint16_t *residual = nullptr);
-
-int gemm_tc_check(cudaStream_t stream);
-// The same GEMM with the dequantised weights in tensor memory (operands swapped: weights are the MMA's M side).
-bool gemm_tm_supported(int M, int K, int N, int group_size);
-int launch_gemm_tm(const uint16_t *A, const int32_t *qweight, const int32_t *qzeros, const uint16_t *scales, uint16_t *C, int M, int K,
-                   int N, cudaStream_t stream, int epilogue = GEMM_EPI_BF16, const uint16_t *residual = nullptr);
-int gemm_tm_check(cudaStream_t stream);
+// Prefill GEMM on CTA pairs (tcgen05, cta_group::2; any M), and the un-quantised bf16 one y = x @ W^T.
+bool gemm_pair_supported(int M, int K, int N, int group_size);
+int launch_gemm_pair(const uint16_t *A, const int32_t *qweight, const int32_t *qzeros, const uint16_t *scales, uint16_t *C, int M, int K,
+                     int N, cudaStream_t stream, int epilogue = GEMM_EPI_BF16, const uint16_t *residual = nullptr);
+bool linear_pair_supported(int M, int K, int N);
+int launch_linear_pair(const uint16_t *x, const uint16_t *W, uint16_t *y, int M, int K, int N, cudaStream_t stream);
+int gemm_pair_check(cudaStream_t stream);
 // Batched-decode GEMM (M <= 128 token rows): stream-K over (column tile, k-block) units, split-K partials through `workspace`.
 bool gemm_decode_supported(int M, int K, int N, int group_size);
 size_t gemm_decode_workspace_bytes(int M, int N);

@@ -4,7 +4,7 @@
 //
 // With this few rows the product is bound by streaming the weights (0.52 B each, used once), like the GEMV,
 // but there are too many rows for mma.sync to keep up, so the multiplies go to tcgen05.  A dequantised bf16
-// tile in shared memory, as in the prefill kernel (awq_gemm_tc.cu), costs 4 bytes of shared-memory traffic per
+// tile in shared memory, as in the first prefill kernel, costs 4 bytes of shared-memory traffic per
 // weight (2 written, 2 read by the MMA): more shared-memory cycles per SM than the weights' share of HBM time.
 // So here the dequantised weights never touch shared memory:
 //

@@ -1,5 +1,5 @@
 // tcgen05 / tensor-memory wrappers shared by the kernels that keep the dequantised weights in tensor memory
-// (awq_gemm_decode.cu, awq_gemm_tm.cu).
+// (awq_gemm_decode.cu, awq_gemm_decode_f8.cu, awq_gemm_pair.cu).
 #pragma once
 
 #include <stdint.h>

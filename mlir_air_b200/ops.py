@@ -112,6 +112,7 @@ def set_deterministic(on: bool):
 
 
 def set_gemm_kernel(mode: str):
+    """"auto", "generic", or the tensor-core kernel where it covers the shape, an error elsewhere ("tc"; "tm" is the same)."""
     _lib.call("awq_b200_set_gemm_kernel", {"auto": 0, "generic": 1, "tc": 2, "tm": 3}[mode])
 
 

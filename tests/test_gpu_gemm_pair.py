@@ -1,0 +1,38 @@
+"""The GEMM on CTA pairs (csrc/awq_gemm_pair.cu) where its tiles, units and plans have their edges, against the oracle."""
+
+import numpy as np
+import pytest
+from ml_dtypes import bfloat16
+
+from oracle import awq_oracle as O
+from gpu_util import dev_weight, randn_bf16, synth_awq, to_dev, to_host
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from mlir_air_b200 import ops as _ops
+    return _ops
+
+
+# unit of 32 token rows, piece of up to 256, two k-blocks of 64 at a time, 256 columns per pair (128 per CTA):
+# one row; a row either side of a unit; of the two-set limit (128); of a piece; rounds and remainders over several column
+# tiles; the second CTA's columns missing, partly missing, complete
+SHAPES = [(1, 128, 32), (31, 128, 128), (33, 256, 160), (128, 384, 256), (129, 384, 288), (256, 128, 512), (257, 640, 96),
+          (300, 256, 2400), (777, 256, 1056), (1030, 128, 4128), (96, 1024, 20480)]
+
+
+@pytest.mark.parametrize("M,K,N", SHAPES)
+def test_int4_edges(ops, M, K, N):
+    qw, qz, s = synth_awq(K, N, 128, seed=M + 5 * N)
+    A, R = randn_bf16((M, K), seed=7), randn_bf16((M, N), seed=9)
+    w = dev_weight(qw, qz, s)
+    acc = A.astype(np.float32) @ O.dequant_to_bf16(qw, qz, s, 128).astype(np.float32)  # the kernel's own operands
+    # f32 sums in another order move a result across a bf16 rounding boundary (2^-8) now and then; a wrong product is 1e-1
+    assert O.rel_l2(to_host(ops.gemm(to_dev(A), w)), acc.astype(bfloat16)) <= 1e-3
+    assert O.rel_l2(to_host(ops.gemm(to_dev(A), w, residual=to_dev(R))), (acc + R.astype(np.float32)).astype(bfloat16)) <= 1e-3
+    gate, up = (acc[:, i::2].astype(bfloat16).astype(np.float32) for i in (0, 1))
+    swiglu = (gate * 0.5 * (np.tanh(gate * 0.5) + 1.0) * up).astype(bfloat16)
+    assert O.rel_l2(to_host(ops.gemm(to_dev(A), w, swiglu=True)), swiglu) <= 2e-3  # two rounded factors
+    ops.gemm_check()
