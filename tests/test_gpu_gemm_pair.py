@@ -1,4 +1,5 @@
-"""The GEMM on CTA pairs (csrc/awq_gemm_pair.cu) where its tiles, units and plans have their edges, against the oracle."""
+"""The GEMM on CTA pairs (csrc/awq_gemm_pair.cu) where its tiles, units and plans have their edges: int4 weights against the
+oracle, bf16 weights against a float64 product."""
 
 import numpy as np
 import pytest
@@ -36,3 +37,40 @@ def test_int4_edges(ops, M, K, N):
     swiglu = (gate * 0.5 * (np.tanh(gate * 0.5) + 1.0) * up).astype(bfloat16)
     assert O.rel_l2(to_host(ops.gemm(to_dev(A), w, swiglu=True)), swiglu) <= 2e-3  # two rounded factors
     ops.gemm_check()
+
+
+@pytest.mark.parametrize("M,K,N", [(16, 8, 8), (17, 72, 136), (64, 136, 250), (129, 2048, 257), (256, 200, 1000), (300, 64, 4104),
+                                   (1025, 192, 520)])
+def test_bf16_edges(ops, M, K, N):
+    """K and N that fill no k-block, no tile and (N % 8 != 0) no 16-byte store."""
+    x, W = randn_bf16((M, K), seed=1), randn_bf16((N, K), seed=2)
+    y = to_host(ops.linear_bf16(to_dev(x), to_dev(W)))
+    ops.gemm_check()
+    ref = (x.astype(np.float64) @ W.astype(np.float64).T).astype(np.float32).astype(bfloat16)
+    assert O.rel_l2(y, ref) <= 1e-3
+
+
+def test_bf16_output_at_any_even_address(ops):
+    import torch
+    x, W = to_dev(randn_bf16((40, 64), seed=1)), to_dev(randn_bf16((136, 64), seed=2))
+    flat = torch.zeros(40 * 136 + 8, dtype=torch.bfloat16, device="cuda")
+    out = flat[1:1 + 40 * 136].view(40, 136)
+    ops.linear_bf16(x, W, out=out)
+    assert torch.equal(out, ops.linear_bf16(x, W)) and not flat[0] and not flat[1 + 40 * 136:].any()
+
+
+def test_runs_back_to_back_are_independent(ops):
+    """Launches overlap by programmatic dependent launch: a chain whose every product reads the one before."""
+    import torch
+    x = to_dev(randn_bf16((200, 512), seed=3))
+    W = to_dev((np.random.default_rng(4).standard_normal((512, 512)) / (1.7 * 512 ** 0.5)).astype(bfloat16))
+    ws = [dev_weight(*synth_awq(512, 512, 128, seed=i)) for i in range(2)]
+    chained, synced = x, x
+    for i in range(6):
+        chained = ops.linear_bf16(ops.gemm(chained, ws[i % 2]), W)
+    for i in range(6):
+        synced = ops.gemm(synced, ws[i % 2])
+        torch.cuda.synchronize()
+        synced = ops.linear_bf16(synced, W)
+        torch.cuda.synchronize()
+    assert torch.equal(chained, synced)
