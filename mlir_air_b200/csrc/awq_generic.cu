@@ -560,12 +560,26 @@ linear_bf16_kernel(const uint16_t *__restrict__ x, const uint16_t *__restrict__ 
 }
 
 // out = bf16(g * sigmoid(g) * u) in f32: the golden form of ffn_swiglu/decode/ffn_decode.py:309-311.
-__global__ void silu_mul_bf16_kernel(const uint16_t *__restrict__ gate, const uint16_t *__restrict__ up,
-                                     uint16_t *__restrict__ out, size_t n) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float g = bf16_bits_to_f32(gate[i]), u = bf16_bits_to_f32(up[i]);
-    out[i] = f32_to_bf16_bits(g * (1.0f / (1.0f + expf(-g))) * u);
+// Eight values a thread where the three buffers allow 16-byte accesses (`vec`); the values past the last whole eight, and everything
+// otherwise, one by one.  512 x 8192: 9.8 -> 5.0 us (the operands come from L2; one value a thread was bound by its
+// 2-byte loads and stores).
+__device__ __forceinline__ float silu_mul_f32(float g, float u) { return g * (1.0f / (1.0f + expf(-g))) * u; }
+__global__ void __launch_bounds__(256)
+silu_mul_bf16_kernel(const uint16_t *__restrict__ gate, const uint16_t *__restrict__ up, uint16_t *__restrict__ out, size_t n, int vec) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, whole = vec ? n >> 3 : 0;
+    if (i < whole) {
+        const uint4 g4 = reinterpret_cast<const uint4 *>(gate)[i], u4 = reinterpret_cast<const uint4 *>(up)[i];
+        const uint32_t g[4] = {g4.x, g4.y, g4.z, g4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
+        uint32_t o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[e] = pack_bf16x2(silu_mul_f32(bf16x2_lo(g[e]), bf16x2_lo(u[e])), silu_mul_f32(bf16x2_hi(g[e]), bf16x2_hi(u[e])));
+        reinterpret_cast<uint4 *>(out)[i] = make_uint4(o[0], o[1], o[2], o[3]);
+        return;
+    }
+    const size_t j = 8 * whole + (i - whole);
+    if (j < n) out[j] = f32_to_bf16_bits(silu_mul_f32(bf16_bits_to_f32(gate[j]), bf16_bits_to_f32(up[j])));
 }
 
 // Per-tile packed buffer (the reference's NPU layout: matvec_int4_packed.py:57-103,
@@ -707,8 +721,10 @@ extern "C" int awq_b200_silu_mul_bf16(const uint16_t *gate, const uint16_t *up, 
                                       awq_stream_t stream) {
     if (n == 0) return AWQ_OK;
     AWQ_REQUIRE(gate && up && out, "silu_mul_bf16: null pointer");
-    silu_mul_bf16_kernel<<<blocks_for(n, 256), 256, 0, as_stream(stream)>>>(gate, up, out, n);
-    return check_cuda(cudaGetLastError(), "silu_mul_bf16 launch");
+    const int vec = aligned16(gate) && aligned16(up) && aligned16(out);
+    return check_cuda(launch_pdl(silu_mul_bf16_kernel, dim3(blocks_for(vec ? n / 8 + n % 8 : n, 256)), dim3(256), 0, as_stream(stream), gate, up,
+                                 out, n, vec),
+                      "silu_mul_bf16 launch");
 }
 
 extern "C" int awq_b200_interleave_gate_up(const int32_t *qw_gate, const int32_t *qz_gate,
