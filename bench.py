@@ -319,7 +319,7 @@ def time_other_configs(a, torch, ops, ffn, peak):
         us = e0.elapsed_time(e1) * 1e3 / (20 * nl)
         g3[str(B)] = dict(_hbm_entry(us, per + 4 * B * H * 2, peak), tokens_per_s=B / (us * 1e-6),
                           path="one launch of the stack kernel for all layers" if st.uses_fused(B) else
-                          ("per layer: RMSNorm + two batched-decode GEMMs (" + ("fp8" if st.uses_gemm_f8(B) else "fp16") + " operands)"
+                          ("per layer: RMSNorm + two batched-decode GEMMs (" + ("fp8" if st.uses_layer(B) or st.uses_gemm_f8(B) else "fp16") + " operands)"
                            if st.uses_gemm(B) else "per-layer kernels"))
     st.check()
     out["ffn_cfg3"] = {"workload": f"decode SwiGLU FFN hidden 4096 / intermediate 11008 with RMSNorm and residual, {nl} distinct "
@@ -360,9 +360,8 @@ def parity_check(a, torch, ops, ffn, group, rank, world):
     # the stack chooses between the two batched-decode GEMMs by the size of a layer: check the one that the timed
     # configuration takes at 32 rows on this many ranks
     f8_min = dict(ffn.DecodeFFNStack.GEMM_F8_MIN_WEIGHTS)
-    if 3 * a.hidden * a.intermediate / world >= f8_min[32]:
-        f8_min = {16: 0, 32: 0}
-    st.GEMM_F8_MIN_WEIGHTS = f8_min
+    if world > 1 and 3 * a.hidden * a.intermediate / world >= f8_min[32]:
+        st.GEMM_F8_MIN_WEIGHTS = {16: 0, 32: 0}
     y_eager = st.step(dev16(x))
     st.load_input(dev16(x))
     y_graph = st.replay(B).clone()
@@ -376,7 +375,8 @@ def parity_check(a, torch, ops, ffn, group, rank, world):
         golden_in.append(O.ffn_layer_A_ref(golden_in[-1], gamma, gate, up, down, gs))
     for l in range(L):
         one = ffn.DecodeFFNStack(layers[l:l + 1], H, max_batch=32, group=group, fused=not a.unfused, peer_push=a.peer_exchange)
-        one.GEMM_F8_MIN_WEIGHTS = f8_min
+        if world > 1:
+            one.GEMM_F8_MIN_WEIGHTS = st.GEMM_F8_MIN_WEIGHTS
         y32_layers.append(one.step(dev16(golden_in[l])))
         one.check()
         del one
@@ -398,7 +398,7 @@ def parity_check(a, torch, ops, ffn, group, rank, world):
                else "per-layer kernels", "oracle": "oracle.awq_oracle.ffn_layer_A_ref, unsharded",
                "batch_32": {"rel_l2": max(max(e32_layers), e32), "rel_l2_per_layer": e32_layers, "rel_l2_end_to_end": e32,
                             "judged": "the chain of all layers, and every layer from the oracle's input of that layer",
-                            "path": ("per layer: RMSNorm + two batched-decode GEMMs (" + ("fp8" if st.uses_gemm_f8(32) else "fp16") + " operands)")
+                            "path": ("per layer: RMSNorm + two batched-decode GEMMs (" + ("fp8" if st.uses_layer(32) or st.uses_gemm_f8(32) else "fp16") + " operands)")
                             if st.uses_gemm(32) else "per-layer kernels"}}
     del st, layers
     return res

@@ -374,6 +374,19 @@ int awq_b200_gemm_decode_f8(const void *A, int a_format, const int32_t *qweight,
                             int swiglu, int M, int K, int N, int group_size, void *workspace,
                             size_t workspace_bytes, awq_stream_t stream);
 
+/* One decode FFN layer for 1 <= M <= 64 token rows on the batched-decode GEMMs (up to 32 rows the one with fp8 operands):
+ *     out [M, H] = bf16(x + down(swiglu(gateup . rmsnorm(x, gamma))))
+ * gate/up column-interleaved [H, 2I], group 128, H and I multiples of 128, H <= 16384; out may be x.  Five launches: the
+ * norm and the SwiGLU are written in the form that the next product reads.  The workspace needs no initialisation
+ * and may be shared with awq_b200_gemm_decode_*. */
+size_t awq_b200_ffn_layer_decode_workspace_bytes(int M, int H, int I);
+int awq_b200_ffn_layer_decode_bf16(const uint16_t *x, const uint16_t *gamma, float eps,
+                                   const int32_t *gateup_qweight, const int32_t *gateup_qzeros,
+                                   const uint16_t *gateup_scales, const int32_t *down_qweight,
+                                   const int32_t *down_qzeros, const uint16_t *down_scales, uint16_t *out, int M,
+                                   int H, int I, int group_size, void *workspace, size_t workspace_bytes,
+                                   awq_stream_t stream);
+
 /* Synchronise `stream` and report whether a tensor-core GEMM (prefill or batched decode) gave up on a
  * bounded device-side wait since the last check (AWQ_ERR_DEVICE_TIMEOUT); the counterpart of
  * xrt.py:204-218. */

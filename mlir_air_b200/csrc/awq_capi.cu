@@ -435,6 +435,26 @@ extern "C" int awq_b200_gemm_decode_f8(const void *A, int a_format, const int32_
                                  workspace, workspace_bytes);
 }
 
+extern "C" size_t awq_b200_ffn_layer_decode_workspace_bytes(int M, int H, int I) { return ffn_layer_workspace_bytes(M, H, I); }
+
+extern "C" int awq_b200_ffn_layer_decode_bf16(const uint16_t *x, const uint16_t *gamma, float eps, const int32_t *gateup_qweight,
+                                              const int32_t *gateup_qzeros, const uint16_t *gateup_scales, const int32_t *down_qweight,
+                                              const int32_t *down_qzeros, const uint16_t *down_scales, uint16_t *out, int M, int H,
+                                              int I, int group_size, void *workspace, size_t workspace_bytes, awq_stream_t stream) {
+    AWQ_REQUIRE(M >= 0 && H > 0 && I > 0 && group_size > 0, "ffn_layer_decode: bad size");
+    if (M == 0) return AWQ_OK;
+    AWQ_REQUIRE(x && gamma && gateup_qweight && gateup_qzeros && gateup_scales && down_qweight && down_qzeros && down_scales && out,
+                "ffn_layer_decode: null pointer");
+    AWQ_REQUIRE(aligned16(x) && aligned16(gamma) && aligned16(gateup_qweight) && aligned16(gateup_qzeros) && aligned16(gateup_scales) &&
+                    aligned16(down_qweight) && aligned16(down_qzeros) && aligned16(down_scales) && aligned16(out) && aligned16(workspace),
+                "ffn_layer_decode: pointers must be 16-byte aligned");
+    if (!ffn_layer_supported(M, H, I, group_size))
+        return set_error(AWQ_ERR_UNSUPPORTED, "ffn_layer_decode: needs M <= 64, group 128, H and I multiples of 128, H <= 16384 "
+                         "(M=%d H=%d I=%d gs=%d)", M, H, I, group_size);
+    return launch_ffn_layer(x, gamma, eps, gateup_qweight, gateup_qzeros, gateup_scales, down_qweight, down_qzeros, down_scales, out,
+                               M, H, I, workspace, workspace_bytes, as_stream(stream));
+}
+
 extern "C" int awq_b200_gemm_decode_bf16(const uint16_t *A, const int32_t *qweight, const int32_t *qzeros,
                                          const uint16_t *scales, const uint16_t *residual, uint16_t *C, int swiglu, int M,
                                          int K, int N, int group_size, void *workspace, size_t workspace_bytes,

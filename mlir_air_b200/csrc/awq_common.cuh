@@ -166,6 +166,13 @@ int launch_gemm_decode_f8(const uint16_t *A, int a_f16, const int32_t *qweight, 
                           uint16_t *C, int M, int K, int N, cudaStream_t stream, int epilogue, const uint16_t *residual, int c_f16,
                           void *workspace, size_t workspace_bytes);
 int gemm_decode_f8_check(cudaStream_t stream);
+// A whole decode FFN layer on the batched-decode GEMMs, up to 64 token rows.
+bool ffn_layer_supported(int M, int H, int I, int group_size);
+size_t ffn_layer_workspace_bytes(int M, int H, int I);
+int launch_ffn_layer(const uint16_t *x, const uint16_t *gamma, float eps, const int32_t *gu_qw, const int32_t *gu_qz, const uint16_t *gu_s,
+                     const int32_t *d_qw, const int32_t *d_qz, const uint16_t *d_s, uint16_t *out, int M, int H, int I, void *workspace,
+                     size_t workspace_bytes, cudaStream_t stream);
+int launch_rmsnorm(const uint16_t *x, const uint16_t *gamma, float eps, uint16_t *out, int out_f16, int B, int K, cudaStream_t stream);
 int gemv_push_arrivals_per_rank(int N);  // arrivals a rank signals per EPI_F32_PUSH launch of N columns
 int launch_tp_reduce_add_rmsnorm(const uint16_t *h, const PeerPartials &parts, unsigned int *flags, int expected,
                                  const uint16_t *gamma, float eps, uint16_t *h_out, uint16_t *normed, int normed_f16, int B,

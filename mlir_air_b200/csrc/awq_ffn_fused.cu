@@ -127,12 +127,6 @@ __device__ __forceinline__ void tma_prefetch_l2_3d(const CUtensorMap *map, int x
                  "r"(z), "l"(policy)
                  : "memory");
 }
-__device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                 "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
-
 struct FusedArgs {
     const FusedLayer *layers;
     int n_layers;

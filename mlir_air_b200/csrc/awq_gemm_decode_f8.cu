@@ -12,16 +12,20 @@
 //    before, two PRMT to bring the same byte of four k into one register, AND / shift-AND to split its two nibbles:
 //    half an instruction per weight, no arithmetic.  tcgen05.mma kind::f8f6f4 multiplies 32 k per instruction, so a
 //    unit takes 8 instructions, not 16.
-//  * The token rows come as e4m3 too, split by a small kernel in front (act_split_kernel): the row is scaled by a power
-//    of two so that its largest magnitude lies in [128, 256), then x = hi + lo / 16 with hi = e4m3(x) and
-//    lo = e4m3(16 (x - hi)).  A bf16 value has 8 significant bits and each piece carries 4, so the split is exact for
-//    every element within 2^-14 of the row's largest (smaller ones keep an absolute error below 2^-22 of it).  The two
-//    pieces are separate MMA columns (N = 2 x rows); inside a 32-k step the k order of both operands is permuted the
+//  * The token rows come as e4m3 too, split into two pieces: scaled by a power of two that brings the largest magnitude into
+//    [128, 256), x = hi + lo / 16 with hi = e4m3(x) and lo = e4m3(16 (x - hi)).  A bf16 value has 8 significant bits and each
+//    piece carries 4, so the split is exact for every element within 2^-14 of the largest (smaller ones keep an absolute
+//    error below 2^-22 of it).  Inside a decode layer (awq_b200_ffn_layer_decode_bf16; GS = true) the power of two belongs to the
+//    row's quantisation group, so the RMSNorm in front of a gate/up product and the second pass of one (SwiGLU) can write
+//    split rows themselves: nobody has to see a whole row first, and a layer has no launch of its own for it.
+//    awq_b200_gemm_decode_f8 (GS = false) is given 16-bit rows: act_split_kernel runs first, with a power of two per row.
+//    The two pieces are separate MMA columns (N = 2 x rows); inside a 32-k step the k order of both operands is permuted the
 //    same way, which costs nothing and lets ldmatrix read conflict-free.
 //  * Zero point and scale never touch the weights.  A unit is one quantisation group, so per weight column n they are
 //    constants of the unit: the MMA leaves P[n, m] = sum_k q x per unit in a fresh accumulator, and eight "promote"
 //    warps (a thread per weight column) fold it into f32 registers:
-//        acc[m] += s (512 P_hi + 32 P_lo - z Sx[m]),   Sx[m] = sum over the group of the split x (from the split kernel)
+//        acc[m] += s (512 P_hi + 32 P_lo - z Sx[m]),   Sx[m] = sum over the group of the split x
+//    (GS: times the group's power of two)
 //    which is exactly sum_k (q - z) s x with the scale applied in f32, as the oracle does: this path rounds no weight.
 //  * Everything else as in awq_gemm_decode.cu: stream-K over (256-column tile, 128 k) units, TMA ring, the sums of a
 //    CTA's share of a tile go to its slot of the workspace and the fix-up launch adds them up (undoing the row's power
@@ -55,9 +59,12 @@ constexpr uint32_t F8_TMEM_COLS = 512;
 template <int NB>
 struct F8Cfg {
     static constexpr int X_BYTES = 2 * NB * DG_GROUP;  // both pieces of every token row, 128 k of one byte
-    static constexpr int SX_OFF = DG_S_BYTES + DG_Z_BYTES;  // the rows' group sums sit behind scales and zeros
-    static constexpr int SX_BYTES = NB * 4;
-    static constexpr int STAGE_BYTES = X_BYTES + DG_W_BYTES + 1024;
+    static constexpr int AUX_BYTES = 1024;
+    // a stage: packed words, token rows, then in AUX_BYTES the rows' group sums (GS: and powers of two), scales, zeros
+    static constexpr int X_OFF = DG_W_BYTES, AUX_OFF = X_OFF + X_BYTES;
+    static constexpr int SX_BYTES = 2 * NB * 4;
+    static constexpr int S_OFF = SX_BYTES, Z_OFF = S_OFF + DG_S_BYTES;  // behind AUX_OFF
+    static constexpr int STAGE_BYTES = X_BYTES + DG_W_BYTES + AUX_BYTES;
     static constexpr int RING_BUDGET = 220 * 1024;
     static constexpr int STAGES = RING_BUDGET / STAGE_BYTES < 8 ? RING_BUDGET / STAGE_BYTES : 8;
     static constexpr int ACC_COLS = 4 * NB;  // two halves x (hi, lo) x rows
@@ -79,7 +86,7 @@ struct F8Cfg {
     static_assert(ACC_COL0 + 2 * ACC_COLS <= (int)F8_TMEM_COLS, "tensor memory budget");
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
     static_assert(STAGE_BYTES % 1024 == 0 && X_BYTES % 1024 == 0, "swizzled tiles need 1024-byte alignment");
-    static_assert(SX_OFF + SX_BYTES <= 1024, "scales, zeros and group sums share one KB");
+    static_assert(S_OFF % 128 == 0 && Z_OFF + DG_Z_BYTES <= AUX_BYTES, "room for scales, zeros and group sums");
 };
 
 __device__ int g_gemm_f8_error;  // 0 = ok; set when a bounded wait gave up
@@ -91,14 +98,14 @@ __device__ __forceinline__ void f8_umma_ta(uint32_t d_tmem, uint32_t a_tmem, uin
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// (d0, d1) += a * (b0, b1): one packed FMA for two token rows
-__device__ __forceinline__ void f8_fma2(float &d0, float &d1, float a, float b0, float b1) {
+// (d0, d1) += (a0, a1) * (b0, b1): one packed FMA for two token rows
+__device__ __forceinline__ void f8_fma2(float &d0, float &d1, float a0, float a1, float b0, float b1) {
     asm("{\n\t.reg .b64 ra, rb, rc;\n\t"
-        "mov.b64 ra, {%2, %2};\n\tmov.b64 rb, {%3, %4};\n\tmov.b64 rc, {%0, %1};\n\t"
+        "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%0, %1};\n\t"
         "fma.rn.f32x2 rc, ra, rb, rc;\n\t"
         "mov.b64 {%0, %1}, rc;\n\t}"
         : "+f"(d0), "+f"(d1)
-        : "f"(a), "f"(b0), "f"(b1));
+        : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
 }
 __device__ __forceinline__ uint32_t f8_prmt(uint32_t a, uint32_t b, uint32_t sel) {
     uint32_t r;
@@ -116,7 +123,7 @@ __host__ __device__ __forceinline__ int f8_k_slot(int k) {
 
 // ---------------------------------------------------------------------------------------------------------------------
 // Split of the token rows.  F8_SPLIT_BLOCKS blocks per (padded) token row: each finds the row's largest magnitude itself (the
-// row comes from L2) and splits its share of the groups.  Output, for rows = 16 or 32 MMA rows:
+// row comes from L2) and splits its share of the groups.  Output, for rows = 16 or 32 MMA rows (the kernel's GS = false):
 //   x8   [K / 128][2 rows][128] bytes: row m = hi piece of token m, row rows + m = lo piece, k permuted inside 32-k steps
 //   sx   [K / 128][rows] f32: sum over the group of hi + lo / 16 (in the row's scaled units)
 //   inv  [rows] f32: the power of two that undoes the row's scaling
@@ -183,10 +190,66 @@ act_split_kernel(const uint16_t *__restrict__ x, int M, int K, int rows, uint8_t
     }
 }
 
+
+// RMSNorm of bf16 rows (the arithmetic of rmsnorm_kernel: f32 sum of squares, f64 reciprocal root, one bf16 rounding), written as
+// split rows.  Several blocks share a row: each forms the row's sum of squares itself (the row comes from L2) and splits one
+// 16-byte chunk a thread, which is the longer part; 16 lanes hold one group.
+constexpr int RS_THREADS = 256, RS_CHUNKS = 8;  // rows up to 16384 elements
+__global__ void __launch_bounds__(RS_THREADS)
+rmsnorm_split_kernel(const uint16_t *__restrict__ h, const uint16_t *__restrict__ gamma, float eps, int K, const SplitRows out) {
+    __shared__ float red[RS_THREADS / 32];
+    pdl_launch_dependents();
+    const int m = blockIdx.x, lane = threadIdx.x & 31, n_chunks = K >> 3, mine = blockIdx.y * RS_THREADS + threadIdx.x;
+    const uint4 gt = mine < n_chunks ? *reinterpret_cast<const uint4 *>(gamma + 8 * mine) : make_uint4(0u, 0u, 0u, 0u);
+    pdl_wait();
+    uint4 t[RS_CHUNKS];
+    float ss = 0.f;
+#pragma unroll
+    for (int c = 0; c < RS_CHUNKS; ++c) {
+        const int ch = threadIdx.x + c * RS_THREADS;
+        t[c] = make_uint4(0u, 0u, 0u, 0u);
+        if (ch < n_chunks) t[c] = *reinterpret_cast<const uint4 *>(h + (size_t)m * K + 8 * ch);
+    }
+    uint4 own = t[0];
+#pragma unroll
+    for (int c = 0; c < RS_CHUNKS; ++c) {
+        if (c == (int)blockIdx.y) own = t[c];
+        const uint32_t w[4] = {t[c].x, t[c].y, t[c].z, t[c].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) ss = fmaf(bf16x2_lo(w[e]), bf16x2_lo(w[e]), ss), ss = fmaf(bf16x2_hi(w[e]), bf16x2_hi(w[e]), ss);
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (lane == 0) red[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    float total = 0.f;
+#pragma unroll
+    for (int w = 0; w < RS_THREADS / 32; ++w) total += red[w];
+    const float rstd = (float)(1.0 / sqrt((double)(total / (float)K) + (double)eps));
+    if (mine >= n_chunks) return;  // n_chunks is a multiple of 16: a group's 16 lanes are in or out together
+    const uint32_t half_mask = 0xFFFFu << (lane & 16);
+    const uint32_t w[4] = {own.x, own.y, own.z, own.w}, gw[4] = {gt.x, gt.y, gt.z, gt.w};
+    float v[8];
+    uint32_t mx = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const uint32_t r = pack_bf16x2((bf16x2_lo(w[e]) * rstd) * bf16x2_lo(gw[e]), (bf16x2_hi(w[e]) * rstd) * bf16x2_hi(gw[e]));
+        v[2 * e] = bf16x2_lo(r), v[2 * e + 1] = bf16x2_hi(r);
+        mx = max(mx, max(__float_as_uint(v[2 * e]) & 0x7FFFFFFFu, __float_as_uint(v[2 * e + 1]) & 0x7FFFFFFFu));
+    }
+    mx = __reduce_max_sync(half_mask, mx);
+    float sum = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) sum += split_pair(out, m, mine >> 4, 8 * (mine & 15) + 2 * e, v[2 * e], v[2 * e + 1], mx);
+#pragma unroll
+    for (int o = 8; o; o >>= 1) sum += __shfl_xor_sync(half_mask, sum, o);
+    if ((lane & 15) == 0) split_finish(out, m, mine >> 4, sum, mx);
+}
+
 // ---------------------------------------------------------------------------------------------------------------------
-template <int NB>
+template <int NB, bool GS>
 __global__ void __launch_bounds__(F8Cfg<NB>::THREADS, 1)
-gemm_decode_f8_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmSx,
+gemm_decode_f8_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmSx, const uint8_t *__restrict__ split,
                       const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmS,
                       const __grid_constant__ CUtensorMap tmZ, int M, int N, int K, int tiles, float *__restrict__ slots,
                       int slots_per_tile, long long wait_limit) {
@@ -208,7 +271,7 @@ gemm_decode_f8_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr uint32_t W_TX_BYTES = DG_W_BYTES + DG_S_BYTES + DG_Z_BYTES;
-    constexpr uint32_t X_TX_BYTES = Cfg::X_BYTES + Cfg::SX_BYTES;
+    constexpr uint32_t X_TX_BYTES = Cfg::X_BYTES + (GS ? Cfg::SX_BYTES : Cfg::SX_BYTES / 2);
     const int KB = K / DG_GROUP;  // units per tile
 
     if (threadIdx.x == 0) {
@@ -240,28 +303,34 @@ gemm_decode_f8_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
     if (warp == 0) {
         // ------------------------------ producer ------------------------------
         if (elect_one()) {
-            tma_prefetch_desc(&tmX);
-            tma_prefetch_desc(&tmSx);
+            if (!GS) {
+                tma_prefetch_desc(&tmX);
+                tma_prefetch_desc(&tmSx);
+            }
             tma_prefetch_desc(&tmW);
             tma_prefetch_desc(&tmS);
             tma_prefetch_desc(&tmZ);
         }
         const uint64_t stream_policy = l2_policy_evict_first();
         auto load_weights = [&](int s, int n0, int g) {
-            const uint32_t st = stage_addr(s) + Cfg::X_BYTES, bar = full_bar(s);
+            const uint32_t st = stage_addr(s), bar = full_bar(s);
             if (elect_one()) {
                 mbar_expect_tx(bar, W_TX_BYTES);
                 tma_load_2d_hint(st, &tmW, n0 / 8, g * DG_GROUP, bar, stream_policy);
-                tma_load_2d(st + DG_W_BYTES, &tmS, n0, g, bar);
-                tma_load_2d(st + DG_W_BYTES + DG_S_BYTES, &tmZ, n0 / 8, g, bar);
+                tma_load_2d(st + Cfg::AUX_OFF + Cfg::S_OFF, &tmS, n0, g, bar);
+                tma_load_2d(st + Cfg::AUX_OFF + Cfg::Z_OFF, &tmZ, n0 / 8, g, bar);
             }
             __syncwarp();
         };
         auto load_rows = [&](int s, int g) {
             if (elect_one()) {
                 mbar_expect_tx(xfull_bar(s), X_TX_BYTES);
-                tma_load_2d(stage_addr(s), &tmX, 0, g * 2 * NB, xfull_bar(s));
-                tma_load_2d(stage_addr(s) + Cfg::X_BYTES + DG_W_BYTES + Cfg::SX_OFF, &tmSx, 0, g, xfull_bar(s));
+                if (GS) {  // one block, as it is to lie in shared memory: a tensor copy less for the producer to issue
+                    bulk_load_1d(stage_addr(s) + Cfg::X_OFF, split + (size_t)g * (Cfg::X_BYTES + Cfg::SX_BYTES), X_TX_BYTES, xfull_bar(s));
+                } else {
+                    tma_load_2d(stage_addr(s) + Cfg::X_OFF, &tmX, 0, g * 2 * NB, xfull_bar(s));
+                    tma_load_2d(stage_addr(s) + Cfg::AUX_OFF, &tmSx, 0, g, xfull_bar(s));
+                }
             }
             __syncwarp();
         };
@@ -289,6 +358,8 @@ gemm_decode_f8_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
             const int s = it % STAGES, round = it / STAGES;
             const int ab = it % Cfg::ABUF, around = it / Cfg::ABUF;
             const int b = it & 1, use = it >> 1;
+            const uint32_t a_tmem = tmem_base + (uint32_t)ab * F8_ABUF_COLS;
+            const uint64_t x_desc = dg_desc_sw128(stage_addr(s) + Cfg::X_OFF);  // K-major 128-byte rows, 32 bytes further per step
             // token rows landed, weight buffer written, accumulator set promoted: three lanes wait side by side
             if (!mbar_wait_multi_warp(use >= 1 ? 3 : 2, xfull_bar(s), round & 1, ready_bar(ab), around & 1, acc_empty(b), (use - 1) & 1,
                                       wait_limit)) {
@@ -297,8 +368,6 @@ gemm_decode_f8_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
             }
             dg_fence_after();
             const uint32_t d_tmem = tmem_base + Cfg::ACC_COL0 + (uint32_t)b * Cfg::ACC_COLS;
-            const uint32_t a_tmem = tmem_base + (uint32_t)ab * F8_ABUF_COLS;
-            const uint64_t x_desc = dg_desc_sw128(stage_addr(s));  // K-major 128-byte rows, 32 bytes further per step
             if (elect_one()) {
 #pragma unroll
                 for (int ks = 0; ks < DG_GROUP / 32; ++ks) {
@@ -333,7 +402,7 @@ gemm_decode_f8_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
                 if (lane == 0) atomicExch(&g_gemm_f8_error, 3);
                 break;
             }
-            const uint32_t st = stage_addr(s) + Cfg::X_BYTES;
+            const uint32_t st = stage_addr(s);
             uint32_t r[4][4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) ldmatrix_x4_trans(r[c], st + w_off + c * 32 * 128);
@@ -393,9 +462,9 @@ gemm_decode_f8_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
                     break;
                 }
                 dg_fence_after();
-                const uint32_t sz = stage_addr(s) + Cfg::X_BYTES + DG_W_BYTES;
-                const float sc = bf16_bits_to_f32((lds32(sz + 2 * (col & ~1)) >> (16 * (col & 1))) & 0xFFFFu);
-                const float z = (float)((lds32(sz + DG_S_BYTES + 4 * (col >> 3)) >> z_shift) & 0xFu);
+                const uint32_t aux = stage_addr(s) + Cfg::AUX_OFF;
+                const float sc = bf16_bits_to_f32((lds32(aux + Cfg::S_OFF + 2 * (col & ~1)) >> (16 * (col & 1))) & 0xFFFFu);
+                const float z = (float)((lds32(aux + Cfg::Z_OFF + 4 * (col >> 3)) >> z_shift) & 0xFu);
                 const float c_hi = 512.f * sc, c_lo = 32.f * sc, c_z = -sc * z;  // a nibble reads as q 2^-9, lo as 16 (x - hi)
                 const uint32_t t_acc = tmem_base + ((uint32_t)(32 * q) << 16) + Cfg::ACC_COL0 + (uint32_t)(b * Cfg::ACC_COLS + h * (2 * NB));
                 // 16 token rows at a time (all 32 at once spill); the accumulator set goes back to the MMA as soon as its last
@@ -413,14 +482,23 @@ gemm_decode_f8_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_cons
                     }
 #pragma unroll
                     for (int j = 0; j < 16; j += 4) {
-                        const uint4 sxv = lds128(sz + Cfg::SX_OFF + 4 * (m0 + j));
+                        const uint4 sxv = lds128(aux + 4 * (m0 + j));
                         const float sx4[4] = {__uint_as_float(sxv.x), __uint_as_float(sxv.y), __uint_as_float(sxv.z), __uint_as_float(sxv.w)};
+                        float in4[4] = {1.f, 1.f, 1.f, 1.f};
+                        if (GS) {
+                            const uint4 inv = lds128(aux + 4 * (NB + m0 + j));
+                            in4[0] = __uint_as_float(inv.x), in4[1] = __uint_as_float(inv.y), in4[2] = __uint_as_float(inv.z), in4[3] = __uint_as_float(inv.w);
+                        }
 #pragma unroll
                         for (int jj = 0; jj < 4; jj += 2) {
-                            float &a0 = acc[m0 + j + jj], &a1 = acc[m0 + j + jj + 1];
-                            f8_fma2(a0, a1, c_z, sx4[jj], sx4[jj + 1]);
-                            f8_fma2(a0, a1, c_lo, __uint_as_float(p_lo[j + jj]), __uint_as_float(p_lo[j + jj + 1]));
-                            f8_fma2(a0, a1, c_hi, __uint_as_float(p_hi[j + jj]), __uint_as_float(p_hi[j + jj + 1]));
+                            float t0 = GS ? c_z * sx4[jj] : acc[m0 + j + jj], t1 = GS ? c_z * sx4[jj + 1] : acc[m0 + j + jj + 1];
+                            if (!GS) f8_fma2(t0, t1, c_z, c_z, sx4[jj], sx4[jj + 1]);
+                            f8_fma2(t0, t1, c_lo, c_lo, __uint_as_float(p_lo[j + jj]), __uint_as_float(p_lo[j + jj + 1]));
+                            f8_fma2(t0, t1, c_hi, c_hi, __uint_as_float(p_hi[j + jj]), __uint_as_float(p_hi[j + jj + 1]));
+                            if (GS)
+                                f8_fma2(acc[m0 + j + jj], acc[m0 + j + jj + 1], in4[jj], in4[jj + 1], t0, t1);
+                            else
+                                acc[m0 + j + jj] = t0, acc[m0 + j + jj + 1] = t1;
                         }
                     }
                 }
@@ -463,51 +541,55 @@ size_t gemm_decode_f8_workspace_bytes(int M, int K, int N) {
     if (M < 1 || N < 1 || K < DG_GROUP) return 0;
     return f8_split_bytes(M, K) + gemm_decode_workspace_bytes(M, N);
 }
+// A decode layer's two products share one workspace: their inputs, then the larger of the slots.  Up to 32 rows the inputs are
+// split rows (the normed rows and the SwiGLU outputs share the memory: the gate/up product is over when its second pass
+// writes), beyond fp16 rows.
+static size_t layer_input_bytes(int M, int H, int I) {
+    const size_t b = M <= F8_MAX_ROWS ? (H > I ? H : I) / DG_GROUP * split_block_bytes(dg_rows(M)) : (size_t)M * ((size_t)H + I) * 2;
+    return (b + 1023) / 1024 * 1024;
+}
+size_t ffn_layer_workspace_bytes(int M, int H, int I) {
+    if (M < 1 || H < DG_GROUP || I < DG_GROUP) return 0;
+    return layer_input_bytes(M, H, I) + gemm_decode_workspace_bytes(M, 2 * I > H ? 2 * I : H);
+}
 
-template <int NB>
-static int launch_f8(const CUtensorMap &tmX, const CUtensorMap &tmSx, const CUtensorMap &tmW, const CUtensorMap &tmS,
-                     const CUtensorMap &tmZ, int M, int N, int K, int tiles, float *slots, int spt, int *ctas_out, cudaStream_t stream) {
+template <int NB, bool GS>
+static int launch_f8(const CUtensorMap &tmX, const CUtensorMap &tmSx, const uint8_t *split, const CUtensorMap &tmW, const CUtensorMap &tmS,
+                     const CUtensorMap &tmZ, int M, int N, int K, int tiles, float *slots, int spt, int ctas, cudaStream_t stream) {
     using Cfg = F8Cfg<NB>;
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(gemm_decode_f8_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
+        attr_err = cudaFuncSetAttribute(gemm_decode_f8_kernel<NB, GS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
     });
     if (attr_err != cudaSuccess) return check_cuda(attr_err, "decode gemm (fp8 operands): shared memory attribute");
-    const int sms = dg_sm_count();
-    const long long U = (long long)tiles * (K / DG_GROUP);
-    const int ctas = (long long)sms < U ? sms : (int)U;
-    *ctas_out = ctas;
-    return check_cuda(launch_pdl(gemm_decode_f8_kernel<NB>, dim3(ctas), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, tmX, tmSx, tmW, tmS, tmZ,
-                                 M, N, K, tiles, slots, spt, wait_limit_cycles()),
+    return check_cuda(launch_pdl(gemm_decode_f8_kernel<NB, GS>, dim3(ctas), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, stream, tmX, tmSx, split, tmW,
+                                 tmS, tmZ, M, N, K, tiles, slots, spt, wait_limit_cycles()),
                       "decode gemm (fp8 operands) launch");
 }
 
-int launch_gemm_decode_f8(const uint16_t *A, int a_f16, const int32_t *qweight, const int32_t *qzeros, const uint16_t *scales,
-                          uint16_t *C, int M, int K, int N, cudaStream_t stream, int epilogue, const uint16_t *residual, int c_f16,
-                          void *workspace, size_t workspace_bytes) {
-    const size_t need = gemm_decode_f8_workspace_bytes(M, K, N);
-    if (!workspace || workspace_bytes < need)
-        return set_error(AWQ_ERR_WORKSPACE, "gemm_decode_f8: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
+// Where a product's token rows are: split with a power of two per group (x8 null), or per row (`sx`, `inv`).
+struct F8Input {
+    const uint8_t *blocks;
+    const uint8_t *x8;
+    const float *sx, *inv;
+};
+// Split rows [M, K] -> product -> epilogue.  `split_out`: a SwiGLU result goes there as split rows (may be the input's memory:
+// the second pass starts when the product is done).
+static int f8_product(const F8Input &in, const int32_t *qweight, const int32_t *qzeros, const uint16_t *scales, uint16_t *C, int M, int K,
+                      int N, cudaStream_t stream, int epilogue, const uint16_t *residual, int c_f16, float *slots, const SplitRows *split_out) {
     const int G = K / DG_GROUP, nb = N / 8, rows = dg_rows(M);
     const int tiles = (N + DG_BN - 1) / DG_BN;
-    uint8_t *x8 = reinterpret_cast<uint8_t *>(workspace);
-    float *sx = reinterpret_cast<float *>(x8 + (size_t)G * 2 * rows * DG_GROUP);
-    float *inv = sx + (size_t)G * rows;
-    float *slots = reinterpret_cast<float *>(x8 + f8_split_bytes(M, K));
+    CUtensorMap tmX = {}, tmSx = {}, tmW, tmS, tmZ;
     int rc;
-    if (a_f16)
-        rc = check_cuda(launch_pdl(act_split_kernel<true>, dim3(rows, F8_SPLIT_BLOCKS), dim3(256), 0, stream, A, M, K, rows, x8, sx, inv), "act split launch");
-    else
-        rc = check_cuda(launch_pdl(act_split_kernel<false>, dim3(rows, F8_SPLIT_BLOCKS), dim3(256), 0, stream, A, M, K, rows, x8, sx, inv), "act split launch");
-    if (rc) return rc;
-    CUtensorMap tmX, tmSx, tmW, tmS, tmZ;
-    if ((rc = encode_tensor_map_2d(&tmX, CU_TENSOR_MAP_DATA_TYPE_UINT8, x8, DG_GROUP, (uint64_t)G * 2 * rows, DG_GROUP, DG_GROUP,
-                                   2 * rows, CU_TENSOR_MAP_SWIZZLE_128B)))
-        return rc;
-    if ((rc = encode_tensor_map_2d(&tmSx, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, sx, rows, G, (uint64_t)rows * 4, rows, 1,
-                                   CU_TENSOR_MAP_SWIZZLE_NONE)))
-        return rc;
+    if (in.x8) {
+        if ((rc = encode_tensor_map_2d(&tmX, CU_TENSOR_MAP_DATA_TYPE_UINT8, in.x8, DG_GROUP, (uint64_t)G * 2 * rows, DG_GROUP, DG_GROUP,
+                                       2 * rows, CU_TENSOR_MAP_SWIZZLE_128B)))
+            return rc;
+        if ((rc = encode_tensor_map_2d(&tmSx, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, in.sx, rows, G, (uint64_t)rows * 4, rows, 1,
+                                       CU_TENSOR_MAP_SWIZZLE_NONE)))
+            return rc;
+    }
     if ((rc = encode_tensor_map_2d(&tmW, CU_TENSOR_MAP_DATA_TYPE_INT32, qweight, nb, K, (uint64_t)nb * 4, DG_BN / 8, DG_GROUP,
                                    CU_TENSOR_MAP_SWIZZLE_128B)))
         return rc;
@@ -518,11 +600,75 @@ int launch_gemm_decode_f8(const uint16_t *A, int a_f16, const int32_t *qweight, 
                                    CU_TENSOR_MAP_SWIZZLE_NONE)))
         return rc;
     const int spt = dg_slots_per_tile(tiles);
-    int ctas = 0;
-    rc = rows == 16 ? launch_f8<16>(tmX, tmSx, tmW, tmS, tmZ, M, N, K, tiles, slots, spt, &ctas, stream)
-                    : launch_f8<32>(tmX, tmSx, tmW, tmS, tmZ, M, N, K, tiles, slots, spt, &ctas, stream);
+    const int sms = dg_sm_count();
+    const long long U = (long long)tiles * G;
+    const int ctas = (long long)sms < U ? sms : (int)U;
+#define F8_LAUNCH(NBV, GSV) launch_f8<NBV, GSV>(tmX, tmSx, in.blocks, tmW, tmS, tmZ, M, N, K, tiles, slots, spt, ctas, stream)
+    if (in.x8)
+        rc = rows == 16 ? F8_LAUNCH(16, false) : F8_LAUNCH(32, false);
+    else
+        rc = rows == 16 ? F8_LAUNCH(16, true) : F8_LAUNCH(32, true);
+#undef F8_LAUNCH
     if (rc) return rc;
-    return launch_gemm_decode_fixup(rows, C, residual, epilogue, c_f16, 1.f, inv, M, N, G, tiles, ctas, slots, spt, stream);
+    return launch_gemm_decode_fixup(rows, C, residual, epilogue, c_f16, in.x8 ? in.inv : nullptr, M, N, G, tiles, ctas, slots, spt, stream, split_out);
+}
+
+int launch_gemm_decode_f8(const uint16_t *A, int a_f16, const int32_t *qweight, const int32_t *qzeros, const uint16_t *scales,
+                          uint16_t *C, int M, int K, int N, cudaStream_t stream, int epilogue, const uint16_t *residual, int c_f16,
+                          void *workspace, size_t workspace_bytes) {
+    const size_t need = gemm_decode_f8_workspace_bytes(M, K, N);
+    if (!workspace || workspace_bytes < need)
+        return set_error(AWQ_ERR_WORKSPACE, "gemm_decode_f8: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
+    const int G = K / DG_GROUP, rows = dg_rows(M);
+    uint8_t *x8 = reinterpret_cast<uint8_t *>(workspace);
+    float *sx = reinterpret_cast<float *>(x8 + (size_t)G * 2 * rows * DG_GROUP);
+    float *inv = sx + (size_t)G * rows;
+    float *slots = reinterpret_cast<float *>(x8 + f8_split_bytes(M, K));
+    int rc;
+    if (a_f16)
+        rc = check_cuda(launch_pdl(act_split_kernel<true>, dim3(rows, F8_SPLIT_BLOCKS), dim3(256), 0, stream, A, M, K, rows, x8, sx, inv), "act split launch");
+    else
+        rc = check_cuda(launch_pdl(act_split_kernel<false>, dim3(rows, F8_SPLIT_BLOCKS), dim3(256), 0, stream, A, M, K, rows, x8, sx, inv), "act split launch");
+    if (rc) return rc;
+    const F8Input in = {nullptr, x8, sx, inv};
+    return f8_product(in, qweight, qzeros, scales, C, M, K, N, stream, epilogue, residual, c_f16, slots, nullptr);
+}
+
+// out [M, H] = bf16(x + down(swiglu(gateup . rmsnorm(x, gamma)))): five launches.  Up to 32 rows on the kernel above, beyond on the
+// 16-bit one.  (A 64-row form of the one above, with the two halves of a tile as its two accumulator sets, measured 215 us per
+// 70B layer against 129: its promote warps' chain is 1,640 cycles per unit, and one half waits for the other.)  Measured
+// in a replayed graph, us per layer at 16 / 32 rows, before (a launch of its own for every split, and the second pass adding
+// its contributors one after another) -> now: hidden 2048, intermediate 8192 26.6 / 30.1 -> 22.1 / 24.4; 4096, 11008 36.9 / 41.1 ->
+// 31.2 / 35.3; 8192, 28672 99 / 105 -> 86 / 99 (in a loop of seconds the last is held at 120 by the power cap either way).  Called
+// without a graph the layer is one call from the host instead of five to seven: 46.9 -> 28.1 us at hidden 2048.
+bool ffn_layer_supported(int M, int H, int I, int group_size) {
+    return gemm_decode_supported(M, H, 2 * I, group_size) && gemm_decode_supported(M, I, H, group_size) &&
+           H <= RS_THREADS * RS_CHUNKS * 8;
+}
+int launch_ffn_layer(const uint16_t *x, const uint16_t *gamma, float eps, const int32_t *gu_qw, const int32_t *gu_qz, const uint16_t *gu_s,
+                     const int32_t *d_qw, const int32_t *d_qz, const uint16_t *d_s, uint16_t *out, int M, int H, int I, void *workspace,
+                     size_t workspace_bytes, cudaStream_t stream) {
+    const size_t need = ffn_layer_workspace_bytes(M, H, I);
+    if (!workspace || workspace_bytes < need)
+        return set_error(AWQ_ERR_WORKSPACE, "ffn_layer_decode: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
+    uint8_t *input = reinterpret_cast<uint8_t *>(workspace), *slots = input + layer_input_bytes(M, H, I);
+    int rc;
+    if (M > F8_MAX_ROWS) {
+        uint16_t *normed = reinterpret_cast<uint16_t *>(input), *inter = normed + (size_t)M * H;
+        const size_t slot_bytes = workspace_bytes - (size_t)(slots - input);
+        if ((rc = launch_rmsnorm(x, gamma, eps, normed, 1, M, H, stream))) return rc;
+        if ((rc = launch_gemm_decode(normed, gu_qw, gu_qz, gu_s, inter, M, H, 2 * I, stream, GEMM_EPI_SWIGLU, nullptr, slots, slot_bytes, 1, 1)))
+            return rc;
+        return launch_gemm_decode(inter, d_qw, d_qz, d_s, out, M, I, H, stream, GEMM_EPI_RESIDUAL, x, slots, slot_bytes, 1, 0);
+    }
+    const SplitRows rows = {input, dg_rows(M)};
+    const F8Input in = {input, nullptr, nullptr, nullptr};
+    rc = check_cuda(launch_pdl(rmsnorm_split_kernel, dim3(M, (H / 8 + RS_THREADS - 1) / RS_THREADS), dim3(RS_THREADS), 0, stream, x, gamma, eps, H, rows),
+                    "rmsnorm split launch");
+    if (rc) return rc;
+    float *slot_words = reinterpret_cast<float *>(slots);
+    if ((rc = f8_product(in, gu_qw, gu_qz, gu_s, nullptr, M, H, 2 * I, stream, GEMM_EPI_SWIGLU, nullptr, 0, slot_words, &rows))) return rc;
+    return f8_product(in, d_qw, d_qz, d_s, out, M, I, H, stream, GEMM_EPI_RESIDUAL, x, 0, slot_words, nullptr);
 }
 
 int gemm_decode_f8_check(cudaStream_t stream) {

@@ -611,6 +611,12 @@ __global__ void repack_C_to_B_sz_kernel(const uint8_t *__restrict__ packed, uint
 
 static inline unsigned blocks_for(size_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
+int launch_rmsnorm(const uint16_t *x, const uint16_t *gamma, float eps, uint16_t *out, int out_f16, int B, int K, cudaStream_t stream) {
+    return check_cuda(launch_pdl(rmsnorm_kernel, dim3(B), dim3(RN_THREADS), 0, stream, x, (const float *)nullptr, gamma, eps,
+                                 (uint16_t *)nullptr, out, K, out_f16),
+                      "rmsnorm launch");
+}
+
 int launch_tp_reduce_add_rmsnorm(const uint16_t *h, const PeerPartials &parts, unsigned int *flags, int expected,
                                  const uint16_t *gamma, float eps, uint16_t *h_out, uint16_t *normed, int normed_f16, int B,
                                  int K, int *err_flag, cudaStream_t stream) {
@@ -631,10 +637,7 @@ extern "C" int awq_b200_rmsnorm_act(const uint16_t *x, const uint16_t *gamma, fl
     AWQ_REQUIRE(out_format == ACT_BF16 || out_format == ACT_F16, "rmsnorm: unknown output format %d", out_format);
     if (B == 0) return AWQ_OK;
     AWQ_REQUIRE(x && gamma && out, "rmsnorm: null pointer");
-    return check_cuda(launch_pdl(rmsnorm_kernel, dim3(B), dim3(256), 0, as_stream(stream), x, (const float *)nullptr,
-                                 gamma, eps, (uint16_t *)nullptr, reinterpret_cast<uint16_t *>(out), K,
-                                 out_format == ACT_F16 ? 1 : 0),
-                      "rmsnorm launch");
+    return launch_rmsnorm(x, gamma, eps, reinterpret_cast<uint16_t *>(out), out_format == ACT_F16 ? 1 : 0, B, K, as_stream(stream));
 }
 
 extern "C" int awq_b200_rmsnorm_bf16(const uint16_t *x, const uint16_t *gamma, float eps, uint16_t *out,

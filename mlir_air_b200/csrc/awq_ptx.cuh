@@ -92,6 +92,12 @@ __device__ __forceinline__ uint64_t l2_policy_evict_last() {
     return p;
 }
 
+// Untiled copy global -> this CTA's shared memory: both addresses and the size multiples of 16 bytes.
+__device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
 // 2-D tiled TMA load global -> this CTA's shared memory, completion counted on `bar`.
 // x is the innermost coordinate in elements; x * element size must be a multiple of 16 bytes.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {

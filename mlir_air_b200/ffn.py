@@ -222,6 +222,16 @@ class DecodeFFNStack:
             return False
         return all(self.gemm_ws.fits_f8(batch, w.K, w.N) for l in self.layers for w in (l.gateup, l.down))
 
+    def uses_layer(self, batch: int) -> bool:
+        """One GPU: each layer is one call (fp8-operand kernel up to 32 rows, 16-bit one beyond).  A stack that was given GEMM_F8_MIN_WEIGHTS of its own runs
+        the separate products that this chooses between."""
+        if self.tp > 1 or "GEMM_F8_MIN_WEIGHTS" in self.__dict__ or not self.uses_gemm(batch):
+            return False
+        fits = getattr(self.gemm_ws, "fits_layer", None)
+        return fits is not None and all(
+            l.gateup.K <= 16384 and l.gateup.N == 2 * l.down.K and l.down.N == l.gateup.K and fits(batch, l.gateup.K, l.down.K)
+            for l in self.layers)
+
     def uses_gemm(self, batch: int) -> bool:
         if batch < self.GEMM_BATCH or batch > 64 or self.gemm_ws is None:
             return False
@@ -233,6 +243,8 @@ class DecodeFFNStack:
     def launches_per_step(self, batch: int) -> int:
         if self.uses_fused(batch):
             return 1
+        if self.uses_layer(batch):
+            return 5 * len(self.layers)
         if self.uses_gemm(batch):
             # norm, and two launches (product, sum of the SMs' shares + epilogue) per GEMM, three with the split of the token
             # rows in front of the fp8-operand kernel; tensor parallel: the norm is fused with the residual add behind the
@@ -274,6 +286,11 @@ class DecodeFFNStack:
                 nxt = self.layers[idx + 1].gamma if idx + 1 < len(self.layers) else None
                 ops.add_rmsnorm(h, partial, nxt, self.eps, h_out=other, normed=normed if nxt is not None else None,
                                 normed_f16=True)
+                h, other = other, h
+            return h
+        if self.uses_layer(B):
+            for l in self.layers:
+                ops.ffn_layer_decode(h, l.gateup, l.down, self.gemm_ws, l.gamma, self.eps, out=other)
                 h, other = other, h
             return h
         if self.uses_gemm(B):

@@ -373,16 +373,20 @@ class GemmDecodeWorkspace:
     columns.  One per stream: calls that share it must not overlap on the GPU."""
 
     def __init__(self, N: int, device="cuda", batch: int = 64, K: int = 0):
-        """`K` > 0 also makes room for the split token rows of `gemm_decode(..., f8=True)` (up to 32 rows of K elements)."""
+        """`K` > 0 also makes room for the split token rows of `gemm_decode(..., f8=True)` and of `ffn_layer_decode`."""
         self.batch, self.N, self.K = int(batch), int(N), int(K)
         lib = _lib.load()
         self.nbytes = int(lib.awq_b200_gemm_decode_workspace_bytes(self.batch, self.N))
         if self.K > 0:
-            self.nbytes = max(self.nbytes, int(lib.awq_b200_gemm_decode_f8_workspace_bytes(min(self.batch, 32), self.K, self.N)))
+            self.nbytes = max(self.nbytes, int(lib.awq_b200_gemm_decode_f8_workspace_bytes(min(self.batch, 32), self.K, self.N)),
+                              int(lib.awq_b200_ffn_layer_decode_workspace_bytes(min(self.batch, 64), self.K, (self.N + 1) // 2)))
         self.buf = torch.empty(self.nbytes, dtype=torch.uint8, device=device)
 
     def fits(self, M, N):
         return int(_lib.load().awq_b200_gemm_decode_workspace_bytes(int(M), int(N))) <= self.nbytes
+
+    def fits_layer(self, M, H, I):
+        return 0 < int(_lib.load().awq_b200_ffn_layer_decode_workspace_bytes(int(M), int(H), int(I))) <= self.nbytes
 
     def fits_f8(self, M, K, N):
         return int(M) <= 32 and 0 < int(_lib.load().awq_b200_gemm_decode_f8_workspace_bytes(int(M), int(K), int(N))) <= self.nbytes
@@ -413,6 +417,21 @@ def gemm_decode(A, w: AwqWeight, ws: GemmDecodeWorkspace, out=None, residual=Non
     _lib.call("awq_b200_gemm_decode_f8" if f8 else "awq_b200_gemm_decode_act", _ptr(A), ACT_F16 if A.dtype == torch.float16 else ACT_BF16, _ptr(w.qweight),
               _ptr(w.qzeros), _ptr(w.scales), _ptr(residual), _ptr(out), OUT_F32 if f32_out else (ACT_F16 if out_f16 else ACT_BF16),
               1 if swiglu else 0, A.shape[0], w.K, w.N, w.group_size, _ptr(ws.buf), ws.nbytes, _stream())
+    return out
+
+
+def ffn_layer_decode(x, w_gateup: AwqWeight, w_down: AwqWeight, ws: GemmDecodeWorkspace, gamma, eps=1e-5, out=None):
+    """out [B, H] = bf16(x + down(swiglu(gateup . rmsnorm(x, gamma)))) for a decode batch of up to 64 rows: one call, five
+    launches (norm, product, SwiGLU, product, residual add)."""
+    x = _x2d(x, w_gateup.K)
+    B, H, I = x.shape[0], w_gateup.K, w_gateup.N // 2
+    if w_down.K != I or w_down.N != H:
+        raise _lib.AwqBackendError(f"down weight must be [{I}, {H}], got [{w_down.K}, {w_down.N}]")
+    if out is None:
+        out = torch.empty((B, H), dtype=torch.bfloat16, device=x.device)
+    _lib.call("awq_b200_ffn_layer_decode_bf16", _ptr(x), _ptr(_want(gamma, torch.bfloat16, "gamma")), float(eps), _ptr(w_gateup.qweight),
+              _ptr(w_gateup.qzeros), _ptr(w_gateup.scales), _ptr(w_down.qweight), _ptr(w_down.qzeros), _ptr(w_down.scales),
+              _ptr(_want(out, torch.bfloat16, "out")), B, H, I, w_gateup.group_size, _ptr(ws.buf), ws.nbytes, _stream())
     return out
 
 

@@ -1,0 +1,58 @@
+"""One decode FFN layer in one call (awq_b200_ffn_layer_decode_bf16) against the numpy oracle: every padded row count, ragged
+column tiles, few and many contributors per tile."""
+import numpy as np
+import pytest
+from ml_dtypes import bfloat16
+
+from oracle import awq_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+# bf16 rounding of the normed rows, of gate and up, of the SwiGLU output and of the result: about 2^-9 / sqrt(3) each
+REL_L2_TOL = 4e-3
+
+
+@pytest.mark.parametrize("B,H,I", [(1, 128, 128), (9, 128, 256), (16, 256, 384), (17, 512, 1408), (32, 384, 640), (33, 512, 1152),
+                                   (48, 1024, 2816), (64, 2048, 5632), (64, 128, 4096), (13, 4096, 128)])
+def test_layer_vs_oracle(B, H, I):
+    import torch
+    from gpu_util import dev_weight, randn_bf16, synth_awq, to_dev, to_host
+    from mlir_air_b200 import ops
+    gate, up = synth_awq(H, I, 128, seed=H + I), synth_awq(H, I, 128, seed=H + I + 1)
+    down = synth_awq(I, H, 128, seed=H + I + 2, scale_lo=0.0005, scale_hi=0.004)
+    gamma = (np.random.default_rng(H).standard_normal(H) * 0.1 + 1.0).astype(bfloat16)
+    wgu, wd = ops.interleave_gate_up(dev_weight(*gate), dev_weight(*up)), dev_weight(*down)
+    ws = ops.GemmDecodeWorkspace(max(2 * I, H), batch=64, K=max(H, I))
+    assert ws.fits_layer(B, H, I)
+    ws.buf.fill_(0xFF)  # NaN in every word: nothing may be read that was not written
+    x = np.asarray(randn_bf16((B, H), seed=B), dtype=np.float32)
+    x[:, ::97] *= 1000.0  # groups and elements of very different size
+    x[0, :64] = 0.0
+    x = x.astype(bfloat16)
+    y = ops.ffn_layer_decode(to_dev(x), wgu, wd, ws, to_dev(gamma))
+    ops.gemm_check()
+    inplace = to_dev(x)
+    ops.ffn_layer_decode(inplace, wgu, wd, ws, to_dev(gamma), out=inplace)
+    ops.gemm_check()
+    assert torch.equal(y, inplace)
+    ref = O.ffn_layer_A_ref(x, gamma, gate, up, down, 128)
+    assert O.rel_l2(to_host(y), ref) <= REL_L2_TOL
+    # without the residual, which is most of the result
+    d, r = to_host(y).astype(np.float32) - x.astype(np.float32), ref.astype(np.float32) - x.astype(np.float32)
+    small = np.ones(H, bool)
+    small[::97] = False
+    assert O.rel_l2(d[:, small], r[:, small]) <= 1e-2
+
+
+def test_layer_refuses():
+    import torch
+    from gpu_util import dev_weight, synth_awq
+    from mlir_air_b200 import ops
+    from mlir_air_b200._lib import AwqBackendError
+    w, d = dev_weight(*synth_awq(128, 512, 128, seed=1)), dev_weight(*synth_awq(256, 128, 128, seed=2))
+    ws = ops.GemmDecodeWorkspace(512, batch=64, K=256)
+    g = torch.ones(128, dtype=torch.bfloat16, device="cuda")
+    with pytest.raises(AwqBackendError):
+        ops.ffn_layer_decode(torch.zeros((65, 128), dtype=torch.bfloat16, device="cuda"), w, d, ws, g)
+    with pytest.raises(AwqBackendError):
+        ops.ffn_layer_decode(torch.zeros((8, 128), dtype=torch.bfloat16, device="cuda"), w, w, ws, g)
