@@ -396,10 +396,24 @@ int awq_b200_gemm_check(awq_stream_t stream);
  * (AWQ_ERR_UNSUPPORTED where it cannot run; automatic takes it wherever it can). */
 int awq_b200_set_gemm_kernel(int mode);
 
+/* awq_b200_gemm_bf16 (no residual, swiglu == 0) and awq_b200_gemm_fused_bf16 with scratch of their own: where the output has too few
+ * tiles for all SMs, K is cut into parts whose f32 sums go through the workspace and are added up in a fixed order by a second
+ * kernel.  awq_b200_gemm_workspace_bytes: what that takes, 0 where it does not pay; with less (or NULL) the product runs
+ * uncut.  The workspace needs no initialisation; calls that share one must not overlap. */
+size_t awq_b200_gemm_workspace_bytes(int M, int K, int N, int group_size);
+int awq_b200_gemm_ws_bf16(const uint16_t *A, const int32_t *qweight, const int32_t *qzeros,
+                          const uint16_t *scales, const uint16_t *residual, uint16_t *C, int swiglu, int M,
+                          int K, int N, int group_size, void *workspace, size_t workspace_bytes,
+                          awq_stream_t stream);
+
 /* ---- bf16 sibling path (un-quantised weights) ----------------------------------------------
  * y bf16 [M, N] = bf16(x[M, K] @ W[N, K]^T): the GEMV/GEMM of ffn_swiglu/decode/ffn_kernels.cc:52-117
  * (matvec_vectorized_bf16_bf16) and ffn_swiglu/prefill/ffn_kernels.cc:55-83 (matmul_bf16).
  * out = bf16(g * sigmoid(g) * u): swiglu_bf16 (ffn_kernels.cc:123-151), golden ffn_decode.py:309-311. */
+/* (with scratch: as awq_b200_gemm_ws_bf16) */
+size_t awq_b200_linear_workspace_bytes(int M, int K, int N);
+int awq_b200_linear_ws_bf16(const uint16_t *x, const uint16_t *W, uint16_t *y, int M, int K, int N, void *workspace,
+                            size_t workspace_bytes, awq_stream_t stream);
 int awq_b200_linear_bf16(const uint16_t *x, const uint16_t *W, uint16_t *y, int M, int K, int N,
                          awq_stream_t stream);
 int awq_b200_silu_mul_bf16(const uint16_t *gate, const uint16_t *up, uint16_t *out, size_t n,

@@ -72,6 +72,10 @@ SIGNATURES = {
     "awq_b200_linear_bf16": (c_int, [_P, _P, _P, c_int, c_int, c_int, _P]),
     "awq_b200_silu_mul_bf16": (c_int, [_P, _P, _P, c_size_t, _P]),
     "awq_b200_gemm_fused_bf16": (c_int, [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P]),
+    "awq_b200_gemm_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
+    "awq_b200_gemm_ws_bf16": (c_int, [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, c_size_t, _P]),
+    "awq_b200_linear_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),
+    "awq_b200_linear_ws_bf16": (c_int, [_P, _P, _P, c_int, c_int, c_int, _P, c_size_t, _P]),
     "awq_b200_gemm_check": (c_int, [_P]),
     "awq_b200_gemm_decode_workspace_bytes": (c_size_t, [c_int, c_int]),
     "awq_b200_gemm_decode_f32": (c_int, [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, _P, c_size_t, _P]),

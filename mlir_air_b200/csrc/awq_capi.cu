@@ -325,9 +325,8 @@ extern "C" int awq_b200_ffn_stack_decode_tp_bf16(const void *plan, int n_layers,
                             &peers);
 }
 
-extern "C" int awq_b200_gemm_bf16(const uint16_t *A, const int32_t *qweight, const int32_t *qzeros,
-                                  const uint16_t *scales, uint16_t *C, int M, int K, int N, int group_size,
-                                  awq_stream_t stream) {
+static int gemm_plain(const uint16_t *A, const int32_t *qweight, const int32_t *qzeros, const uint16_t *scales, uint16_t *C, int M, int K,
+                      int N, int group_size, void *workspace, size_t workspace_bytes, awq_stream_t stream) {
     AWQ_REQUIRE(M >= 0 && K >= 0 && N >= 0 && group_size > 0, "gemm: negative size or group_size <= 0");
     AWQ_REQUIRE(N % 8 == 0, "gemm: N (%d) must be a multiple of 8", N);
     AWQ_REQUIRE(K % group_size == 0, "gemm: K (%d) must be a multiple of group_size (%d)", K, group_size);
@@ -341,13 +340,19 @@ extern "C" int awq_b200_gemm_bf16(const uint16_t *A, const int32_t *qweight, con
     if (mode >= 2 && !tc_ok)
         return set_error(AWQ_ERR_UNSUPPORTED, "gemm: tensor-core kernel does not cover M=%d K=%d N=%d gs=%d", M, K, N,
                          group_size);
-    if (mode != 1 && tc_ok) return launch_gemm_pair(A, qweight, qzeros, scales, C, M, K, N, as_stream(stream));
+    if (mode != 1 && tc_ok)
+        return launch_gemm_pair(A, qweight, qzeros, scales, C, M, K, N, as_stream(stream), GEMM_EPI_BF16, nullptr, workspace, workspace_bytes);
     return launch_gemm_generic(A, qweight, qzeros, scales, C, M, K, N, group_size, as_stream(stream));
 }
+extern "C" int awq_b200_gemm_bf16(const uint16_t *A, const int32_t *qweight, const int32_t *qzeros,
+                                  const uint16_t *scales, uint16_t *C, int M, int K, int N, int group_size,
+                                  awq_stream_t stream) {
+    return gemm_plain(A, qweight, qzeros, scales, C, M, K, N, group_size, nullptr, 0, stream);
+}
 
-extern "C" int awq_b200_gemm_fused_bf16(const uint16_t *A, const int32_t *qweight, const int32_t *qzeros,
-                                        const uint16_t *scales, const uint16_t *residual, uint16_t *C, int swiglu, int M,
-                                        int K, int N, int group_size, awq_stream_t stream) {
+static int gemm_fused(const uint16_t *A, const int32_t *qweight, const int32_t *qzeros, const uint16_t *scales, const uint16_t *residual,
+                      uint16_t *C, int swiglu, int M, int K, int N, int group_size, void *workspace, size_t workspace_bytes,
+                      awq_stream_t stream) {
     AWQ_REQUIRE(M >= 0 && K > 0 && N > 0 && group_size > 0, "gemm_fused: bad size");
     AWQ_REQUIRE(!(swiglu && residual), "gemm_fused: SwiGLU and residual do not combine");
     if (M == 0) return AWQ_OK;
@@ -358,7 +363,23 @@ extern "C" int awq_b200_gemm_fused_bf16(const uint16_t *A, const int32_t *qweigh
         return set_error(AWQ_ERR_UNSUPPORTED, "gemm_fused: needs the tensor-core kernel (group 128, K %% 128 == 0, N %% 32 == 0; "
                          "M=%d K=%d N=%d gs=%d)", M, K, N, group_size);
     const int epi = swiglu ? GEMM_EPI_SWIGLU : (residual ? GEMM_EPI_RESIDUAL : GEMM_EPI_BF16);
-    return launch_gemm_pair(A, qweight, qzeros, scales, C, M, K, N, as_stream(stream), epi, residual);
+    return launch_gemm_pair(A, qweight, qzeros, scales, C, M, K, N, as_stream(stream), epi, residual, workspace, workspace_bytes);
+}
+extern "C" int awq_b200_gemm_fused_bf16(const uint16_t *A, const int32_t *qweight, const int32_t *qzeros,
+                                        const uint16_t *scales, const uint16_t *residual, uint16_t *C, int swiglu, int M,
+                                        int K, int N, int group_size, awq_stream_t stream) {
+    return gemm_fused(A, qweight, qzeros, scales, residual, C, swiglu, M, K, N, group_size, nullptr, 0, stream);
+}
+
+extern "C" size_t awq_b200_gemm_workspace_bytes(int M, int K, int N, int group_size) {
+    return M >= 1 && K > 0 && N > 0 && group_size > 0 && gemm_pair_supported(M, K, N, group_size) ? gemm_pair_workspace_bytes(M, K, N) : 0;
+}
+extern "C" int awq_b200_gemm_ws_bf16(const uint16_t *A, const int32_t *qweight, const int32_t *qzeros, const uint16_t *scales,
+                                     const uint16_t *residual, uint16_t *C, int swiglu, int M, int K, int N, int group_size,
+                                     void *workspace, size_t workspace_bytes, awq_stream_t stream) {
+    AWQ_REQUIRE(aligned16(workspace), "gemm: the workspace must be 16-byte aligned");
+    return residual || swiglu ? gemm_fused(A, qweight, qzeros, scales, residual, C, swiglu, M, K, N, group_size, workspace, workspace_bytes, stream)
+                              : gemm_plain(A, qweight, qzeros, scales, C, M, K, N, group_size, workspace, workspace_bytes, stream);
 }
 
 extern "C" int awq_b200_gemm_check(awq_stream_t stream) {

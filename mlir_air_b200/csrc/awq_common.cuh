@@ -147,9 +147,13 @@ enum GemmEpilogue : int { GEMM_EPI_BF16 = 0, GEMM_EPI_RESIDUAL = 1, GEMM_EPI_SWI
 // Prefill GEMM on CTA pairs (tcgen05, cta_group::2; any M), and the un-quantised bf16 one y = x @ W^T.
 bool gemm_pair_supported(int M, int K, int N, int group_size);
 int launch_gemm_pair(const uint16_t *A, const int32_t *qweight, const int32_t *qzeros, const uint16_t *scales, uint16_t *C, int M, int K,
-                     int N, cudaStream_t stream, int epilogue = GEMM_EPI_BF16, const uint16_t *residual = nullptr);
+                     int N, cudaStream_t stream, int epilogue = GEMM_EPI_BF16, const uint16_t *residual = nullptr, void *workspace = nullptr,
+                     size_t workspace_bytes = 0);  // a workspace lets K be cut into parts where the tiles leave SMs idle
+size_t gemm_pair_workspace_bytes(int M, int K, int N);
 bool linear_pair_supported(int M, int K, int N);
-int launch_linear_pair(const uint16_t *x, const uint16_t *W, uint16_t *y, int M, int K, int N, cudaStream_t stream);
+int launch_linear_pair(const uint16_t *x, const uint16_t *W, uint16_t *y, int M, int K, int N, cudaStream_t stream, void *workspace = nullptr,
+                       size_t workspace_bytes = 0);
+size_t linear_pair_workspace_bytes(int M, int K, int N);
 int gemm_pair_check(cudaStream_t stream);
 // Batched-decode GEMM (M <= 128 token rows): stream-K over (column tile, k-block) units, split-K partials through `workspace`.
 bool gemm_decode_supported(int M, int K, int N, int group_size);

@@ -10,6 +10,9 @@
 // dequantised weights as a shared-memory tile / in tensor memory with 192-row tiles dealt round-robin):
 //   128 x 4096 x 14336   35 -> 20      512 x 4096 x 14336   59 -> 50     2048 x 4096 x 14336   202 -> 173 (1.39 PFLOP/s)
 //   128 x 14336 x 4096  105 -> 50      777 x 14336 x 4096  106 -> 73     4096 x 8192 x 57344  3350 -> 3090
+// With scratch from the caller, K cut into parts (uncut -> cut, second pass included): 128 x 14336 x 4096 49 -> 23, 256 x 8192 x 2048
+// 31 -> 18, 65 x 4096 x 4096 19 -> 13.5; bf16 weights 512 x 8192 x 2048 34 -> 24.  Letting the next launch start early (programmatic
+// dependent launch) takes 1 to 2 us off each launch in a row: 96 x 512 x 1024 8.2 -> 6.0.
 //
 //   int4   the weights are dequantised into tensor memory (ldmatrix.trans -> LOP3 / bf16x2 -> tcgen05.st), each CTA its
 //          own 128 columns; four groups of four dequant warps take alternate k-blocks and hold a finished k-block in
@@ -94,8 +97,10 @@ struct PairMaps {
 // ones per column tile): the pairs of a round share token rows and weights in L2.  What does not fill a round is cut
 // evenly: units from `base` on, counted column tile by column tile, one contiguous range per pair, where a cut closer than
 // `snap` units to a column tile's edge moves there.
+// With S > 1, P pairs share the plane S times: the pairs of part s multiply the s-th part of K and leave f32 sums, which a
+// second kernel adds up (gemm_pair_sum_kernel).
 struct PairPlan {
-    int P, R, C, max_units, sets, waves, NT, base, snap;
+    int P, R, C, max_units, sets, waves, NT, base, snap, S;
     __host__ __device__ int cut(int p) const {
         const int v = base + (int)((long long)p * ((long long)R * C - base) / P), r = v % R;
         if (r == 0) return v;
@@ -267,9 +272,11 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, uint16_t *__restrict__ C
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = gp_cluster_rank();
-    const int KB = (K + 2 * GP_BK - 1) / (2 * GP_BK) * 2;  // k-blocks, multiplied two at a time
+    const int KB2 = (K + 2 * GP_BK - 1) / (2 * GP_BK);  // k-blocks are multiplied two at a time
+    const int pair = (int)(blockIdx.x >> 1), part = pair / plan.P;
+    const int kb_first = part * KB2 / plan.S * 2, KB = (part + 1) * KB2 / plan.S * 2 - kb_first;  // this pair's part of K
     constexpr int ACC_STRIDE = W4 ? GP_ABUF_COL0 / 2 : 256;  // columns between two accumulator sets
-    PairWalk walk((int)(blockIdx.x >> 1), plan);
+    PairWalk walk(pair - part * plan.P, plan);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < stages; ++s) mbar_init(full_bar(s), 1);
@@ -318,18 +325,19 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, uint16_t *__restrict__ C
                     break;
                 }
                 const uint32_t st = stage_addr(s), bar = full0 + 8u * s;
+                const int k0 = (kb_first + kb) * GP_BK;
                 if (elect_one()) {
                     if (W4) {
-                        const int g = kb * GP_BK / GP_GROUP;
+                        const int g = k0 / GP_GROUP;
                         mbar_expect_tx(bar, tx);
-                        tma_load_2d(st + x_bytes, &maps.w, n0 / 8, kb * GP_BK, bar);
+                        tma_load_2d(st + x_bytes, &maps.w, n0 / 8, k0, bar);
                         tma_load_2d(st + x_bytes + Cfg::W_BYTES, &maps.s, n0, g, bar);
                         tma_load_2d(st + x_bytes + Cfg::W_BYTES + Cfg::S_BYTES, &maps.z, n0 / 8, g, bar);
-                        tma_load_2d(st, mx, kb * GP_BK, m0, bar);
+                        tma_load_2d(st, mx, k0, m0, bar);
                     } else {
                         if (rank == 0) mbar_expect_tx(full_bar(s), 2 * tx);  // both CTAs' copies are counted on the leader's barrier
-                        gp_tma_load_2d_pair(st, mx, kb * GP_BK, m0, bar);
-                        gp_tma_load_2d_pair(st + x_bytes, &maps.w, kb * GP_BK, n0, bar);
+                        gp_tma_load_2d_pair(st, mx, k0, m0, bar);
+                        gp_tma_load_2d_pair(st + x_bytes, &maps.w, k0, n0, bar);
                     }
                 }
                 __syncwarp();
@@ -470,6 +478,31 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, uint16_t *__restrict__ C
             const int set = acc_sets == 2 ? piece & 1 : 0, use = acc_sets == 2 ? piece >> 1 : piece;
             const int rows = walk.units * GP_UNIT, m_base = walk.unit * GP_UNIT, n0 = walk.tile * GP_BN + (int)rank * GP_HALF;
             const int valid = M - m_base < rows ? M - m_base : rows;
+            if (plan.S > 1) {
+                // this part's sums as they are: a lane per column, 16 token rows at a time
+                const bool full = mbar_wait_bounded(acc_full(set), use & 1, wait_limit);
+                if (!__all_sync(0xffffffffu, full)) {
+                    if (lane == 0) atomicExch(&g_gemm_pair_error, 5);
+                    break;
+                }
+                dg_fence_after();
+                const int n_pad = plan.C * GP_BN;
+                float *out = reinterpret_cast<float *>(C) + ((size_t)part * M + m_base) * n_pad + n0 + 32 * q + (W4 ? dg_lane_column(lane) : lane);
+                const uint32_t acc = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(set * ACC_STRIDE);
+                for (int t = th * (rows / 2); t < (th + 1) * (rows / 2); t += 16) {
+                    uint32_t v[16];
+                    dg_tmem_ld_32x32b_x16(acc + (uint32_t)t, v);
+                    dg_tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if (t + i < valid) __stcg(out + (size_t)(t + i) * n_pad, __uint_as_float(v[i]));
+                }
+                dg_fence_before();
+                __syncwarp();
+                if (lane == 0) gp_arrive_cluster(acc_empty_leader[set]);
+                ++piece;
+                continue;
+            }
             if (epi == GEMM_EPI_RESIDUAL) {
                 // the residual tile goes through the staging tile in the order the accumulators will have there
                 named_bar_sync(1, ET);  // the previous piece has left the staging tile
@@ -601,15 +634,57 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, uint16_t *__restrict__ C
     }
 }
 
+// Second pass of a product whose K was cut into S parts: four columns of a token row a thread, the parts' sums in their order, then
+// the epilogue (the rounding points of the kernel above).
+constexpr int GP_MAX_PARTS = 8;
+__global__ void __launch_bounds__(256)
+gemm_pair_sum_kernel(const float *__restrict__ parts, int S, uint16_t *__restrict__ C, const uint16_t *__restrict__ R, int epi, int M, int N,
+                     int n_pad) {
+    pdl_wait();
+    const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
+    const int quads = n_pad >> 2, m = (int)(idx / quads), n = 4 * (int)(idx - (long long)m * quads);
+    if (m >= M || n >= N) return;
+    const float *src = parts + (size_t)m * n_pad + n;
+    float4 v[GP_MAX_PARTS];
+#pragma unroll
+    for (int s = 0; s < GP_MAX_PARTS; ++s)
+        if (s < S) v[s] = __ldcg(reinterpret_cast<const float4 *>(src + (size_t)s * M * n_pad));
+    float4 sum = v[0];
+#pragma unroll
+    for (int s = 1; s < GP_MAX_PARTS; ++s)
+        if (s < S) sum.x += v[s].x, sum.y += v[s].y, sum.z += v[s].z, sum.w += v[s].w;
+    if (epi == GEMM_EPI_SWIGLU) {  // (N is a multiple of 32)
+        *reinterpret_cast<uint32_t *>(C + (size_t)m * (N >> 1) + (n >> 1)) =
+            (uint32_t)swiglu_bits(sum.x, sum.y) | ((uint32_t)swiglu_bits(sum.z, sum.w) << 16);
+        return;
+    }
+    uint16_t *out = C + (size_t)m * N + n;
+    if (epi == GEMM_EPI_RESIDUAL) {
+        const uint2 r = *reinterpret_cast<const uint2 *>(R + (size_t)m * N + n);
+        sum.x += bf16x2_lo(r.x), sum.y += bf16x2_hi(r.x), sum.z += bf16x2_lo(r.y), sum.w += bf16x2_hi(r.y);
+    }
+    const uint2 o = make_uint2(gp_cvt_bf16x2(sum.x, sum.y), gp_cvt_bf16x2(sum.z, sum.w));
+    if ((N & 3) == 0 && ((size_t)C & 7) == 0) {
+        *reinterpret_cast<uint2 *>(out) = o;
+    } else {
+        for (int i = 0; i < 4 && n + i < N; ++i) out[i] = (uint16_t)((i < 2 ? o.x : o.y) >> (16 * (i & 1)));
+    }
+}
+
 // ---------------------------------------------------------------------------------------------
 // The longest pair's time for a plan, in cycles.  Measured with clock64 per k-block of 64: 69 cycles per unit of 32 token
 // rows (64 at the tensor pipe's peak), but not less than about 370 with int4 weights (the chain of a dequant group: fetch
-// 240, arithmetic 630, tensor-memory store 200, over four groups) and 265 with bf16 ones (loads in flight: a narrow piece's
-// stage is mostly weights).  A piece's drain is exposed where there is one accumulator set: 2,600 cycles.
-static long long pair_cost(const PairPlan &pl, int KB, bool w4) {
-    const int floor_cycles = w4 ? 370 : 265, drain = pl.sets == 2 ? 600 : 3000;
+// 240, arithmetic 630, tensor-memory store 200, over four groups) and 280 plus 35 per unit with bf16 ones (its bytes at the
+// 59 bytes per cycle and SM that L2 delivers: a narrow piece's stage is mostly weights).  A piece's drain is exposed where there is one accumulator set: 2,600 cycles.  Parts of K: their sums
+// cross L2 twice, and the second pass is a launch.
+static size_t pair_parts_bytes(int M, int N, int S) { return (size_t)S * M * ((N + GP_BN - 1) / GP_BN * GP_BN) * 4; }
+constexpr size_t GP_PARTS_MAX_BYTES = 64u << 20;  // about half of L2
+static long long pair_cost(const PairPlan &pl, int KB_all, bool w4, int M) {
+    const int KB = (KB_all / 2 + pl.S - 1) / pl.S * 2;
+    const int floor_cycles = w4 ? 370 : 280, floor_unit = w4 ? 0 : 35, drain = pl.sets == 2 ? 600 : 3000;
     auto segment = [&](int len, int n) -> long long {  // `len` units of one column tile in n pieces
-        const long long kblock = 69 * len > n * floor_cycles ? 69 * len : n * floor_cycles;
+        const long long least = (long long)n * floor_cycles + (long long)len * floor_unit;
+        const long long kblock = 69 * len > least ? 69 * len : least;
         return KB * kblock + (long long)n * drain;
     };
     auto cut_up = [&](int len) -> long long { return len <= 0 ? 0 : segment(len, (len + pl.max_units - 1) / pl.max_units); };
@@ -622,72 +697,92 @@ static long long pair_cost(const PairPlan &pl, int KB, bool w4) {
         if (t > worst) worst = t;
         a = b;
     }
-    return worst + pl.waves * segment((pl.R + pl.NT - 1) / pl.NT, 1);
+    const long long parts = pl.S > 1 ? 6000 + (long long)pl.S * M * pl.C * GP_BN * 4 / 1000 : 0;
+    return worst + pl.waves * segment((pl.R + pl.NT - 1) / pl.NT, 1) + parts;
 }
 
 // The cheapest plan for a shape: a pure function of the sizes; the last shapes are remembered, the search takes microseconds.
 template <bool W4>
-static PairPlan pair_plan(int M, int N, int K, int pairs) {
+static PairPlan pair_plan(int M, int N, int K, int all_pairs, bool may_split) {
     struct Memo {
-        int M = 0, N = 0, K = 0, pairs = 0;
+        int M = 0, N = 0, K = 0, pairs = 0, split = 0;
         PairPlan plan;
     };
-    thread_local Memo memo[16];
-    Memo &m = memo[(unsigned)(M * 31 + N * 7 + K) % 16];
-    if (m.M == M && m.N == N && m.K == K && m.pairs == pairs) return m.plan;
+    thread_local Memo memo[64];
+    Memo &m = memo[(((unsigned)M * 2654435761u ^ (unsigned)N * 2246822519u ^ (unsigned)K * 3266489917u) >> 27) * 2 + may_split];
+    if (m.M == M && m.N == N && m.K == K && m.pairs == all_pairs && m.split == may_split) return m.plan;
     PairPlan pl, best_plan;
     pl.R = (M + GP_UNIT - 1) / GP_UNIT;
     pl.C = (N + GP_BN - 1) / GP_BN;
     const int KB = (K + 2 * GP_BK - 1) / (2 * GP_BK) * 2;
     long long best = -1;
     auto consider = [&] {
-        const long long c = pair_cost(pl, KB, W4);
+        const long long c = pair_cost(pl, KB, W4, M);
         if (best < 0 || c < best) best = c, best_plan = pl;
     };
     const int nt_min = (pl.R + GP_MAX_UNITS - 1) / GP_MAX_UNITS;
-    for (pl.NT = nt_min; pl.NT <= pl.R && pl.NT < nt_min + 4; ++pl.NT) {
-        const int tiles = pl.NT * pl.C;
-        pl.max_units = (pl.R + pl.NT - 1) / pl.NT;  // of a tile, and of a piece of what is cut evenly
-        pl.sets = !W4 || pl.max_units <= GP_MAX_UNITS / 2 ? 2 : 1;
-        pl.P = tiles < pairs ? tiles : pairs;
-        for (int back = 0; back < 2 && back <= tiles / pl.P; ++back) {  // rounds; the rest is cut evenly
-            pl.waves = tiles / pl.P - back;
-            const int t = pl.waves * pl.P;
-            pl.base = t / pl.NT * pl.R + t % pl.NT * pl.R / pl.NT;
-            if (t == tiles) {
-                pl.snap = 0;
-                consider();
-                continue;
+    // parts of K: of eight k-blocks at least, and not where the plane alone gives every pair two pieces
+    for (pl.S = 1; pl.S == 1 || (may_split && pl.S <= GP_MAX_PARTS && KB >= 8 * pl.S && pl.C * nt_min < 2 * all_pairs &&
+                                 pair_parts_bytes(M, N, pl.S) <= GP_PARTS_MAX_BYTES);
+         pl.S += pl.S < 4 ? 1 : 2) {
+        const int pairs = all_pairs / pl.S;
+        for (pl.NT = nt_min; pl.NT <= pl.R && pl.NT < nt_min + 4; ++pl.NT) {
+            const int tiles = pl.NT * pl.C;
+            pl.max_units = (pl.R + pl.NT - 1) / pl.NT;  // of a tile, and of a piece of what is cut evenly
+            pl.sets = !W4 || pl.max_units <= GP_MAX_UNITS / 2 ? 2 : 1;
+            pl.P = tiles < pairs ? tiles : pairs;
+            for (int back = 0; back < 2 && back <= tiles / pl.P; ++back) {  // rounds; the rest is cut evenly
+                pl.waves = tiles / pl.P - back;
+                const int t = pl.waves * pl.P;
+                pl.base = t / pl.NT * pl.R + t % pl.NT * pl.R / pl.NT;
+                if (t == tiles) {
+                    pl.snap = 0;
+                    consider();
+                    continue;
+                }
+                if (pl.S > 1) continue;  // parts of whole tiles only (512 x 8192 x 2048 bf16: 20.8 us so, 23.1 in three parts cut evenly)
+                for (int sn : {0, 2, pl.R}) {
+                    pl.snap = sn;
+                    consider();
+                }
             }
-            for (int sn : {0, 2, pl.R}) {
-                pl.snap = sn;
-                consider();
-            }
-        }
-        if (tiles < pairs && pl.R * pl.C > tiles) {  // fewer tiles than pairs: cut everything evenly over all pairs
-            pl.P = pl.R * pl.C < pairs ? pl.R * pl.C : pairs;
-            pl.waves = pl.base = 0;
-            for (int sn : {0, 2}) {
-                pl.snap = sn;
-                consider();
+            if (pl.S == 1 && tiles < pairs && pl.R * pl.C > tiles) {  // fewer tiles than pairs: cut everything evenly over all pairs
+                pl.P = pl.R * pl.C < pairs ? pl.R * pl.C : pairs;
+                pl.waves = pl.base = 0;
+                for (int sn : {0, 2}) {
+                    pl.snap = sn;
+                    consider();
+                }
             }
         }
     }
-    m.M = M, m.N = N, m.K = K, m.pairs = pairs, m.plan = best_plan;
+    m.M = M, m.N = N, m.K = K, m.pairs = all_pairs, m.split = may_split, m.plan = best_plan;
     return best_plan;
 }
 
+static int pair_count() {
+    const int sms = device_sm_count();
+    return (sms > 0 ? sms : 148) / 2;
+}
+// Scratch that lets the plan cut K: 0 where it would not.
+template <bool W4>
+static size_t pair_workspace_bytes(int M, int K, int N) {
+    const PairPlan plan = pair_plan<W4>(M, N, K, pair_count(), true);
+    return plan.S > 1 ? pair_parts_bytes(M, N, plan.S) : 0;
+}
+size_t gemm_pair_workspace_bytes(int M, int K, int N) { return pair_workspace_bytes<true>(M, K, N); }
+size_t linear_pair_workspace_bytes(int M, int K, int N) { return pair_workspace_bytes<false>(M, K, N); }
+
 template <bool W4>
 static int launch_pair(const uint16_t *A, const void *w, const int32_t *qzeros, const uint16_t *scales, uint16_t *C, int M, int K, int N,
-                       cudaStream_t stream, int epilogue, const uint16_t *residual) {
+                       cudaStream_t stream, int epilogue, const uint16_t *residual, void *workspace, size_t workspace_bytes) {
     using Cfg = PairCfg<W4>;
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] { attr_err = cudaFuncSetAttribute(gemm_pair_kernel<W4>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM_MAX); });
     if (attr_err != cudaSuccess) return check_cuda(attr_err, "pair gemm: shared memory attribute");
-    int sms = device_sm_count();
-    if (sms <= 0) sms = 148;
-    const PairPlan plan = pair_plan<W4>(M, N, K, sms / 2);
+    PairPlan plan = pair_plan<W4>(M, N, K, pair_count(), workspace != nullptr);
+    if (plan.S > 1 && workspace_bytes < pair_parts_bytes(M, N, plan.S)) plan = pair_plan<W4>(M, N, K, pair_count(), false);
     const PairLayout lay = pair_layout<W4>(plan.max_units);
     const size_t smem = 1024 + (size_t)lay.stages * lay.stage_bytes + Cfg::BAR_BYTES + (size_t)lay.staging_rows * GP_STAGING_STRIDE;
     PairMaps maps;
@@ -712,21 +807,27 @@ static int launch_pair(const uint16_t *A, const void *w, const int32_t *qzeros, 
                                        CU_TENSOR_MAP_SWIZZLE_128B)))
             return rc;
     }
-    const cudaError_t e = launch_pdl(gemm_pair_kernel<W4>, dim3(2 * plan.P), dim3(Cfg::THREADS), smem, stream, maps, C, residual, epilogue,
-                                     M, N, K, plan, wait_limit_cycles());
-    return check_cuda(e, "pair gemm launch");
+    uint16_t *out = plan.S > 1 ? reinterpret_cast<uint16_t *>(workspace) : C;
+    const cudaError_t e = launch_pdl(gemm_pair_kernel<W4>, dim3(2 * plan.P * plan.S), dim3(Cfg::THREADS), smem, stream, maps, out, residual,
+                                     epilogue, M, N, K, plan, wait_limit_cycles());
+    if (e != cudaSuccess || plan.S == 1) return check_cuda(e, "pair gemm launch");
+    const int n_pad = plan.C * GP_BN;
+    return check_cuda(launch_pdl(gemm_pair_sum_kernel, dim3((unsigned)(((long long)M * (n_pad / 4) + 255) / 256)), dim3(256), 0, stream,
+                                 reinterpret_cast<const float *>(workspace), plan.S, C, residual, epilogue, M, N, n_pad),
+                      "pair gemm sum launch");
 }
 
 bool gemm_pair_supported(int M, int K, int N, int group_size) {
     return group_size == GP_GROUP && K % GP_GROUP == 0 && N % 32 == 0 && M >= 1 && K > 0 && N > 0 && device_is_sm100();
 }
 int launch_gemm_pair(const uint16_t *A, const int32_t *qweight, const int32_t *qzeros, const uint16_t *scales, uint16_t *C, int M, int K,
-                     int N, cudaStream_t stream, int epilogue, const uint16_t *residual) {
-    return launch_pair<true>(A, qweight, qzeros, scales, C, M, K, N, stream, epilogue, residual);
+                     int N, cudaStream_t stream, int epilogue, const uint16_t *residual, void *workspace, size_t workspace_bytes) {
+    return launch_pair<true>(A, qweight, qzeros, scales, C, M, K, N, stream, epilogue, residual, workspace, workspace_bytes);
 }
 bool linear_pair_supported(int M, int K, int N) { return K % 8 == 0 && M >= 1 && K > 0 && N > 0 && device_is_sm100(); }
-int launch_linear_pair(const uint16_t *x, const uint16_t *W, uint16_t *y, int M, int K, int N, cudaStream_t stream) {
-    return launch_pair<false>(x, W, nullptr, nullptr, y, M, K, N, stream, GEMM_EPI_BF16, nullptr);
+int launch_linear_pair(const uint16_t *x, const uint16_t *W, uint16_t *y, int M, int K, int N, cudaStream_t stream, void *workspace,
+                       size_t workspace_bytes) {
+    return launch_pair<false>(x, W, nullptr, nullptr, y, M, K, N, stream, GEMM_EPI_BF16, nullptr, workspace, workspace_bytes);
 }
 
 int gemm_pair_check(cudaStream_t stream) {

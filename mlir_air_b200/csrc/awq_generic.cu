@@ -705,8 +705,18 @@ extern "C" int awq_b200_rope_halfsplit_bf16(const uint16_t *x, size_t x_stride, 
     return check_cuda(cudaGetLastError(), "rope launch");
 }
 
+extern "C" size_t awq_b200_linear_workspace_bytes(int M, int K, int N) {
+    return M >= 16 && K > 0 && N > 0 && linear_pair_supported(M, K, N) ? linear_pair_workspace_bytes(M, K, N) : 0;
+}
+
 extern "C" int awq_b200_linear_bf16(const uint16_t *x, const uint16_t *W, uint16_t *y, int M, int K, int N,
                                     awq_stream_t stream) {
+    return awq_b200_linear_ws_bf16(x, W, y, M, K, N, nullptr, 0, stream);
+}
+
+extern "C" int awq_b200_linear_ws_bf16(const uint16_t *x, const uint16_t *W, uint16_t *y, int M, int K, int N, void *workspace,
+                                       size_t workspace_bytes, awq_stream_t stream) {
+    AWQ_REQUIRE(aligned16(workspace), "linear_bf16: the workspace must be 16-byte aligned");
     AWQ_REQUIRE(M >= 0 && K > 0 && N >= 0, "linear_bf16: bad size");
     AWQ_REQUIRE(K % 8 == 0, "linear_bf16: K (%d) must be a multiple of 8", K);
     if (M == 0 || N == 0) return AWQ_OK;
@@ -714,7 +724,8 @@ extern "C" int awq_b200_linear_bf16(const uint16_t *x, const uint16_t *W, uint16
     AWQ_REQUIRE(aligned16(x) && aligned16(W), "linear_bf16: x and W must be 16-byte aligned");
     // From 16 rows on a tensor-core GEMM (one pass over the weights whatever M), below a warp per output column: the line
     // lies where the warps' second pass over the weights (8 rows each) costs as much as the GEMM's pipeline fill.
-    if (M >= 16 && linear_pair_supported(M, K, N)) return launch_linear_pair(x, W, y, M, K, N, as_stream(stream));
+    if (M >= 16 && linear_pair_supported(M, K, N))
+        return launch_linear_pair(x, W, y, M, K, N, as_stream(stream), workspace, workspace_bytes);
     dim3 grid((N + 7) / 8, (M + LB_ROWS - 1) / LB_ROWS);
     linear_bf16_kernel<<<grid, 256, 0, as_stream(stream)>>>(x, W, y, M, K, N);
     return check_cuda(cudaGetLastError(), "linear_bf16 launch");

@@ -29,6 +29,16 @@ def _want(t: torch.Tensor, dtype, name: str):
     return t
 
 
+def _aligned16(*tensors):
+    return not any(t is not None and t.data_ptr() & 15 for t in tensors)
+
+
+def _parts(size_fn: str, device, *dims):
+    """Scratch that the kernel chosen for these sizes asks for, from torch's stream-ordered allocator; None where it needs none."""
+    n = int(getattr(_lib.load(), size_fn)(*dims))
+    return torch.empty(n, dtype=torch.uint8, device=device) if n else None
+
+
 @dataclass
 class AwqWeight:
     """One AWQ-quantised linear layer in HF AutoAWQ layout (layout A), resident on a GPU.
@@ -358,11 +368,21 @@ def gemm(A, w: AwqWeight, out=None, residual=None, swiglu=False):
         _want(out, torch.bfloat16, "out")
         if residual is not None:
             _want(residual, torch.bfloat16, "residual")
+        ws = _parts("awq_b200_gemm_workspace_bytes", out.device, A.shape[0], w.K, w.N, w.group_size)
+        if ws is not None:
+            _lib.call("awq_b200_gemm_ws_bf16", _ptr(A), _ptr(w.qweight), _ptr(w.qzeros), _ptr(w.scales), _ptr(residual), _ptr(out),
+                      1 if swiglu else 0, A.shape[0], w.K, w.N, w.group_size, _ptr(ws), ws.numel(), _stream())
+            return out
         _lib.call("awq_b200_gemm_fused_bf16", _ptr(A), _ptr(w.qweight), _ptr(w.qzeros), _ptr(w.scales), _ptr(residual),
                   _ptr(out), 1 if swiglu else 0, A.shape[0], w.K, w.N, w.group_size, _stream())
         return out
     if out is None:
         out = torch.empty((A.shape[0], w.N), dtype=torch.bfloat16, device=A.device)
+    ws = _parts("awq_b200_gemm_workspace_bytes", out.device, A.shape[0], w.K, w.N, w.group_size)
+    if ws is not None:
+        _lib.call("awq_b200_gemm_ws_bf16", _ptr(A), _ptr(w.qweight), _ptr(w.qzeros), _ptr(w.scales), None, _ptr(out), 0, A.shape[0],
+                  w.K, w.N, w.group_size, _ptr(ws), ws.numel(), _stream())
+        return out
     _lib.call("awq_b200_gemm_bf16", _ptr(A), _ptr(w.qweight), _ptr(w.qzeros), _ptr(w.scales), _ptr(out), A.shape[0],
               w.K, w.N, w.group_size, _stream())
     return out
@@ -463,6 +483,11 @@ def linear_bf16(x, W, out=None):
     x2 = x.view(1, -1) if x.dim() == 1 else x
     if out is None:
         out = torch.empty((x2.shape[0], W.shape[0]), dtype=torch.bfloat16, device=x.device)
+    ws = _parts("awq_b200_linear_workspace_bytes", out.device, x2.shape[0], x2.shape[1], W.shape[0])
+    if ws is not None:
+        _lib.call("awq_b200_linear_ws_bf16", _ptr(x2), _ptr(W), _ptr(out), x2.shape[0], x2.shape[1], W.shape[0], _ptr(ws), ws.numel(),
+                  _stream())
+        return out
     _lib.call("awq_b200_linear_bf16", _ptr(x2), _ptr(W), _ptr(out), x2.shape[0], x2.shape[1], W.shape[0], _stream())
     return out
 

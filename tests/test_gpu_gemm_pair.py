@@ -74,3 +74,45 @@ def test_runs_back_to_back_are_independent(ops):
         synced = ops.linear_bf16(synced, W)
         torch.cuda.synchronize()
     assert torch.equal(chained, synced)
+
+
+# K cut into parts: one piece per part, ragged last tiles and rows, parts of unequal length, N that takes scalar stores
+@pytest.mark.parametrize("M,K,N", [(65, 4096, 4096), (16, 8192, 256), (100, 2048, 544), (300, 8192, 2048), (257, 14336, 1056), (40, 1152, 32)])
+def test_int4_k_parts(ops, M, K, N):
+    qw, qz, s = synth_awq(K, N, 128, seed=M + N)
+    A, R = randn_bf16((M, K), seed=7), randn_bf16((M, N), seed=9)
+    w = dev_weight(qw, qz, s)
+    acc = A.astype(np.float64) @ O.dequant_to_bf16(qw, qz, s, 128).astype(np.float64)
+    assert O.rel_l2(to_host(ops.gemm(to_dev(A), w)), acc.astype(np.float32).astype(bfloat16)) <= 1e-3
+    assert O.rel_l2(to_host(ops.gemm(to_dev(A), w, residual=to_dev(R))), (acc + R.astype(np.float64)).astype(np.float32).astype(bfloat16)) <= 1e-3
+    gate, up = (acc[:, i::2].astype(np.float32).astype(bfloat16).astype(np.float32) for i in (0, 1))
+    swiglu = (gate * 0.5 * (np.tanh(gate * 0.5) + 1.0) * up).astype(bfloat16)
+    assert O.rel_l2(to_host(ops.gemm(to_dev(A), w, swiglu=True)), swiglu) <= 2e-3
+    ops.gemm_check()
+
+
+@pytest.mark.parametrize("M,K,N", [(512, 8192, 2048), (64, 4096, 250), (17, 8200, 257), (300, 1100 * 8, 520)])
+def test_bf16_k_parts(ops, M, K, N):
+    x, W = randn_bf16((M, K), seed=1), randn_bf16((N, K), seed=2)
+    y = to_host(ops.linear_bf16(to_dev(x), to_dev(W)))
+    ops.gemm_check()
+    assert O.rel_l2(y, (x.astype(np.float64) @ W.astype(np.float64).T).astype(np.float32).astype(bfloat16)) <= 1e-3
+
+
+def test_k_parts_without_a_workspace(ops):
+    """The entry point without scratch, and one that is given too little, run the product uncut."""
+    import torch
+    from mlir_air_b200 import _lib
+    M, K, N = 128, 14336, 4096
+    w, A = dev_weight(*synth_awq(K, N, 128, seed=3)), to_dev(randn_bf16((M, K), seed=4))
+    need = _lib.load().awq_b200_gemm_workspace_bytes(M, K, N, 128)
+    assert need > 0
+    cut, whole, small = ops.gemm(A, w), torch.empty((M, N), dtype=torch.bfloat16, device="cuda"), torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+    args = (A.data_ptr(), w.qweight.data_ptr(), w.qzeros.data_ptr(), w.scales.data_ptr())
+    stream = torch.cuda.current_stream().cuda_stream
+    _lib.call("awq_b200_gemm_bf16", *args, whole.data_ptr(), M, K, N, 128, stream)
+    ws = torch.empty(need - 16, dtype=torch.uint8, device="cuda")
+    _lib.call("awq_b200_gemm_ws_bf16", *args, None, small.data_ptr(), 0, M, K, N, 128, ws.data_ptr(), ws.numel(), stream)
+    ops.gemm_check()
+    assert torch.equal(whole, small)
+    assert (cut.double() - whole.double()).norm() <= 1e-3 * whole.double().norm()
