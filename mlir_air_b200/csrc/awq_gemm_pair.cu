@@ -297,6 +297,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, uint16_t *__restrict__ C
     gp_cluster_sync();  // the peer's barriers are initialised
     dg_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_launch_dependents();
     pdl_wait();
 
     if (warp == 0 || (warp > 1 && warp <= Cfg::PRODUCERS)) {
@@ -640,6 +641,7 @@ constexpr int GP_MAX_PARTS = 8;
 __global__ void __launch_bounds__(256)
 gemm_pair_sum_kernel(const float *__restrict__ parts, int S, uint16_t *__restrict__ C, const uint16_t *__restrict__ R, int epi, int M, int N,
                      int n_pad) {
+    pdl_launch_dependents();
     pdl_wait();
     const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
     const int quads = n_pad >> 2, m = (int)(idx / quads), n = 4 * (int)(idx - (long long)m * quads);
