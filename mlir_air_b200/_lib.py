@@ -124,4 +124,6 @@ def check(status: int, what: str = ""):
 
 def call(name: str, *args):
     """Call `name` and raise AwqBackendError unless it returns AWQ_OK."""
-    check(getattr(load(), name)(*args), name)
+    status = getattr(_lib or load(), name)(*args)
+    if status != AWQ_OK:
+        check(status, name)

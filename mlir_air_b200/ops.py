@@ -15,8 +15,13 @@ def _ptr(t: Optional[torch.Tensor]):
     return None if t is None else t.data_ptr()
 
 
+# torch.cuda.current_stream().cuda_stream without the Stream object in between (3.1 -> 0.2 us, of about 13 for an operator call
+# whose kernel takes 3); the operators' tensors exist, so CUDA is initialised
+_raw_stream, _device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+
+
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_device())
 
 
 def _want(t: torch.Tensor, dtype, name: str):
