@@ -374,6 +374,16 @@ int awq_b200_gemm_decode_f8(const void *A, int a_format, const int32_t *qweight,
                             int swiglu, int M, int K, int N, int group_size, void *workspace,
                             size_t workspace_bytes, awq_stream_t stream);
 
+/* y [B, N] = x [B, K] @ W (+ residual), as awq_b200_gemv_bf16 / awq_b200_gemv_f32 (y_f32 != 0) give it, for 9 <= B <= 64 bf16 rows, on
+ * the fp8-operand kernel in passes of up to 32 rows.  No value is out of range (an infinity or a NaN shows in the output).
+ * awq_b200_gemv_rows_workspace_bytes: scratch, 0 where this does not apply or another kernel was asked for
+ * (awq_b200_set_decode_kernel).  The workspace needs no initialisation; calls that share one must not overlap. */
+size_t awq_b200_gemv_rows_workspace_bytes(int B, int K, int N, int group_size);
+int awq_b200_gemv_rows_bf16(const uint16_t *x, const int32_t *qweight, const int32_t *qzeros,
+                            const uint16_t *scales, const uint16_t *residual, void *y, int y_f32, int B, int K,
+                            int N, int group_size, void *workspace, size_t workspace_bytes,
+                            awq_stream_t stream);
+
 /* One decode FFN layer for 1 <= M <= 64 token rows on the batched-decode GEMMs (up to 32 rows the one with fp8 operands):
  *     out [M, H] = bf16(x + down(swiglu(gateup . rmsnorm(x, gamma))))
  * gate/up column-interleaved [H, 2I], group 128, H and I multiples of 128, H <= 16384; out may be x.  Five launches: the

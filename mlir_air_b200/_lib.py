@@ -82,6 +82,8 @@ SIGNATURES = {
     "awq_b200_gemm_decode_act": (c_int, [_P, c_int, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_size_t, _P]),
     "awq_b200_gemm_decode_f8_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),
     "awq_b200_gemm_decode_f8": (c_int, [_P, c_int, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, c_int, _P, c_size_t, _P]),
+    "awq_b200_gemv_rows_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
+    "awq_b200_gemv_rows_bf16": (c_int, [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, c_size_t, _P]),
     "awq_b200_ffn_layer_decode_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),
     "awq_b200_ffn_layer_decode_bf16": (c_int, [_P, _P, c_float] + [_P] * 7 + [c_int, c_int, c_int, c_int, _P, c_size_t, _P]),
     "awq_b200_gemm_decode_bf16": (c_int, [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_int, c_int, _P, c_size_t, _P]),

@@ -456,6 +456,25 @@ extern "C" int awq_b200_gemm_decode_f8(const void *A, int a_format, const int32_
                                  workspace, workspace_bytes);
 }
 
+extern "C" size_t awq_b200_gemv_rows_workspace_bytes(int B, int K, int N, int group_size) {
+    if (B < 9 || B > 64 || K <= 0 || N <= 0 || group_size <= 0 || g_decode_mode.load() != 0 ||
+        !gemm_decode_f8_supported(B < 32 ? B : 32, K, N, group_size))
+        return 0;
+    return gemv_rows_workspace_bytes(B, K, N);
+}
+extern "C" int awq_b200_gemv_rows_bf16(const uint16_t *x, const int32_t *qweight, const int32_t *qzeros, const uint16_t *scales,
+                                       const uint16_t *residual, void *y, int y_f32, int B, int K, int N, int group_size,
+                                       void *workspace, size_t workspace_bytes, awq_stream_t stream) {
+    AWQ_REQUIRE(x && qweight && qzeros && scales && y && workspace, "gemv_rows: null pointer");
+    AWQ_REQUIRE(aligned16(x) && aligned16(qweight) && aligned16(qzeros) && aligned16(scales) && aligned16(residual) && aligned16(y) &&
+                    aligned16(workspace), "gemv_rows: pointers must be 16-byte aligned");
+    AWQ_REQUIRE(!(y_f32 && residual), "gemv_rows: the f32 output takes no residual");
+    if (B < 9 || B > 64 || K <= 0 || N <= 0 || !gemm_decode_f8_supported(B < 32 ? B : 32, K, N, group_size))
+        return set_error(AWQ_ERR_UNSUPPORTED, "gemv_rows: needs 9 to 64 rows, group 128, K %% 128 == 0, N %% 32 == 0 (B=%d K=%d N=%d gs=%d)", B,
+                         K, N, group_size);
+    return launch_gemv_rows(x, qweight, qzeros, scales, residual, y, y_f32, B, K, N, workspace, workspace_bytes, as_stream(stream));
+}
+
 extern "C" size_t awq_b200_ffn_layer_decode_workspace_bytes(int M, int H, int I) { return ffn_layer_workspace_bytes(M, H, I); }
 
 extern "C" int awq_b200_ffn_layer_decode_bf16(const uint16_t *x, const uint16_t *gamma, float eps, const int32_t *gateup_qweight,

@@ -170,6 +170,9 @@ int launch_gemm_decode_f8(const uint16_t *A, int a_f16, const int32_t *qweight, 
                           uint16_t *C, int M, int K, int N, cudaStream_t stream, int epilogue, const uint16_t *residual, int c_f16,
                           void *workspace, size_t workspace_bytes);
 int gemm_decode_f8_check(cudaStream_t stream);
+size_t gemv_rows_workspace_bytes(int M, int K, int N);
+int launch_gemv_rows(const uint16_t *x, const int32_t *qweight, const int32_t *qzeros, const uint16_t *scales, const uint16_t *residual,
+                     void *y, int y_f32, int M, int K, int N, void *workspace, size_t workspace_bytes, cudaStream_t stream);
 // A whole decode FFN layer on the batched-decode GEMMs, up to 64 token rows.
 bool ffn_layer_supported(int M, int H, int I, int group_size);
 size_t ffn_layer_workspace_bytes(int M, int H, int I);

@@ -191,6 +191,26 @@ act_split_kernel(const uint16_t *__restrict__ x, int M, int K, int rows, uint8_t
 }
 
 
+// bf16 rows as split rows (GS = true): a warp per (token row, group), four consecutive values a lane.
+__global__ void __launch_bounds__(256)
+rows_split_kernel(const uint16_t *__restrict__ x, int M, int K, const SplitRows out) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int G = K / DG_GROUP, lane = threadIdx.x & 31, idx = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int m = idx / G, g = idx - m * G;
+    if (m >= M) return;
+    const uint2 q = *reinterpret_cast<const uint2 *>(x + (size_t)m * K + (size_t)g * DG_GROUP + 4 * lane);
+    const float v[4] = {bf16x2_lo(q.x), bf16x2_hi(q.x), bf16x2_lo(q.y), bf16x2_hi(q.y)};
+    uint32_t mx = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) mx = max(mx, __float_as_uint(v[e]) & 0x7FFFFFFFu);
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    float sum = split_pair(out, m, g, 4 * lane, v[0], v[1], mx) + split_pair(out, m, g, 4 * lane + 2, v[2], v[3], mx);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) split_finish(out, m, g, sum, mx);
+}
+
 // RMSNorm of bf16 rows (the arithmetic of rmsnorm_kernel: f32 sum of squares, f64 reciprocal root, one bf16 rounding), written as
 // split rows.  Several blocks share a row: each forms the row's sum of squares itself (the row comes from L2) and splits one
 // 16-byte chunk a thread, which is the longer part; 16 lanes hold one group.
@@ -632,6 +652,37 @@ int launch_gemm_decode_f8(const uint16_t *A, int a_f16, const int32_t *qweight, 
     if (rc) return rc;
     const F8Input in = {nullptr, x8, sx, inv};
     return f8_product(in, qweight, qzeros, scales, C, M, K, N, stream, epilogue, residual, c_f16, slots, nullptr);
+}
+
+// y [M, N] = x @ W (+ residual) for 9 to 64 bf16 rows, in passes of up to 32: what awq_b200_gemv_rows_bf16 runs.  (The multi-row
+// GEMV kernel feeds mma.sync eight rows at a time from a decoded fragment: 32 rows of 4096 x 11008 25.2 us, here 18.7; 64 of
+// 8192 x 28672 143, here 84.)
+size_t gemv_rows_workspace_bytes(int M, int K, int N) {
+    const int rows = dg_rows(M < F8_MAX_ROWS ? M : F8_MAX_ROWS);
+    return (K / DG_GROUP * split_block_bytes(rows) + 1023) / 1024 * 1024 + gemm_decode_workspace_bytes(rows, N);
+}
+int launch_gemv_rows(const uint16_t *x, const int32_t *qweight, const int32_t *qzeros, const uint16_t *scales, const uint16_t *residual,
+                     void *y, int y_f32, int M, int K, int N, void *workspace, size_t workspace_bytes, cudaStream_t stream) {
+    const size_t need = gemv_rows_workspace_bytes(M, K, N);
+    if (!workspace || workspace_bytes < need)
+        return set_error(AWQ_ERR_WORKSPACE, "gemv_rows: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
+    uint8_t *blocks = reinterpret_cast<uint8_t *>(workspace);
+    const int passes = (M + F8_MAX_ROWS - 1) / F8_MAX_ROWS;
+    for (int p = 0; p < passes; ++p) {
+        const int m0 = p * M / passes, m = (p + 1) * M / passes - m0, rows = dg_rows(m);
+        float *slots = reinterpret_cast<float *>(blocks + (K / DG_GROUP * split_block_bytes(rows) + 1023) / 1024 * 1024);
+        const SplitRows split = {blocks, rows};
+        int rc = check_cuda(launch_pdl(rows_split_kernel, dim3((unsigned)((m * (K / DG_GROUP) + 7) / 8)), dim3(256), 0, stream,
+                                       x + (size_t)m0 * K, m, K, split),
+                            "row split launch");
+        if (rc) return rc;
+        const F8Input in = {blocks, nullptr, nullptr, nullptr};
+        uint16_t *out = y_f32 ? reinterpret_cast<uint16_t *>(reinterpret_cast<float *>(y) + (size_t)m0 * N) : reinterpret_cast<uint16_t *>(y) + (size_t)m0 * N;
+        rc = f8_product(in, qweight, qzeros, scales, out, m, K, N, stream, y_f32 ? GEMM_EPI_F32 : (residual ? GEMM_EPI_RESIDUAL : GEMM_EPI_BF16),
+                        residual ? residual + (size_t)m0 * N : nullptr, 0, slots, nullptr);
+        if (rc) return rc;
+    }
+    return AWQ_OK;
 }
 
 // out [M, H] = bf16(x + down(swiglu(gateup . rmsnorm(x, gamma)))): five launches.  Up to 32 rows on the kernel above, beyond on the

@@ -106,6 +106,7 @@ class Workspace:
         """Synchronise and raise if a device-side wait timed out."""
         with torch.cuda.device(self.buf.device):
             _lib.call("awq_b200_workspace_check", self.buf.data_ptr(), _stream())
+            _lib.call("awq_b200_gemm_check", _stream())  # gemv of more than 8 rows: the batched-decode GEMM's waits
 
 
 ACT_BF16, ACT_F16, OUT_F32 = 0, 1, 2
@@ -159,6 +160,12 @@ def _x2d(x, K, f16=False):
     return x
 
 
+# From how many weights on bf16 gemv calls of 9 to 16 and of 17 to 64 rows take the fp8-operand GEMM: it is three launches where the
+# multi-row GEMV kernel is two, and 3 us more for the host.  Measured per call, multi-row GEMV / GEMM: 32 rows, 45 M weights
+# 25.2 / 18.7 us; 64 rows, 235 M 143 / 84; 24 rows, 15 M 18.2 / 18.9; 16 rows, 45 M 16.0 / 18.6, and per 70B layer in a graph 108 / 86.
+GEMV_ROWS_MIN_WEIGHTS = {16: 100e6, 64: 32e6}
+
+
 def gemv(x, w: AwqWeight, ws: Workspace, residual=None, out=None, f32_out=False, x_f16=False):
     """y [B, N] = x [B, K] @ W (+ residual); bf16 with one rounding, or the f32 partial.
     x is bf16, or fp16 (the library's internal activation format) with x_f16."""
@@ -171,6 +178,12 @@ def gemv(x, w: AwqWeight, ws: Workspace, residual=None, out=None, f32_out=False,
     if residual is not None:
         _want(residual, torch.bfloat16, "residual")
     _want(out, torch.float32 if f32_out else torch.bfloat16, "out")
+    if B > 8 and not x_f16 and w.K * w.N >= GEMV_ROWS_MIN_WEIGHTS[16 if B <= 16 else 64] and _aligned16(x, w.qweight, w.qzeros, w.scales, residual, out):
+        scratch = _parts("awq_b200_gemv_rows_workspace_bytes", out.device, B, w.K, w.N, w.group_size)
+        if scratch is not None:
+            _lib.call("awq_b200_gemv_rows_bf16", _ptr(x), _ptr(w.qweight), _ptr(w.qzeros), _ptr(w.scales), _ptr(residual), _ptr(out),
+                      1 if f32_out else 0, B, w.K, w.N, w.group_size, _ptr(scratch), scratch.numel(), _stream())
+            return out
     _lib.call("awq_b200_gemv_act", _ptr(x), ACT_F16 if x_f16 else ACT_BF16, _ptr(w.qweight), _ptr(w.qzeros),
               _ptr(w.scales), _ptr(residual), _ptr(out), 1 if f32_out else 0, B, w.K, w.N, w.group_size, _ptr(ws.buf),
               ws.nbytes, _stream())
