@@ -74,9 +74,11 @@ constexpr int FF_MAX_LAYERS = 1024;  // 2 claim words per layer in shared memory
 // (it grows by four per layer), and per k-group of the gate/up projection (128 hidden values) how many of its two
 // 64-column sub-strips (two per layer); then one f32 sum of squares per (layer boundary, batch row).
 constexpr size_t FF_STATE_OFF = SK_WS_END;
-constexpr size_t FF_STATE_HEADER = 64;
+// Words that one SM counts up while others poll them lie in sectors of their own (side by side, 70B layer: 74.0 -> 73.1 us).
+constexpr size_t FF_STATE_HEADER = 512;
+constexpr int FF_DONE_STRIDE = 64, FF_READY_STRIDE = 8;
 constexpr int FF_READY_WORDS = 1024;  // >= SK_MAX_GROUPS, per direction
-constexpr size_t FF_READY_BYTES = 2 * FF_READY_WORDS * sizeof(int);
+constexpr size_t FF_READY_BYTES = 2 * FF_READY_WORDS * FF_READY_STRIDE * sizeof(int);
 __host__ __device__ constexpr size_t ff_state_bytes(int n_layers) {
     return FF_STATE_HEADER + FF_READY_BYTES + (size_t)(n_layers + 1) * 8 * sizeof(float);
 }
@@ -231,12 +233,12 @@ ffn_fused_kernel(const __grid_constant__ CUtensorMap tmXi, const __grid_constant
     // phase 0: gate/up, K = H, N = 2I; phase 1: down, K = I, N = H
     const int G0 = H / SK_GROUP, V0 = (2 * I + SK_STRIP - 1) / SK_STRIP;
     const int G1 = I / SK_GROUP, V1 = (H + SK_STRIP - 1) / SK_STRIP;
-    int *done_gu = a.state, *done_d = a.state + 1;
+    int *done_gu = a.state, *done_d = a.state + FF_DONE_STRIDE;
     const bool tp = a.tp_n > 1;
     // tensor parallel: exchanges so far on these buffers (all launches run the same number of layers); every
     // warp reads the count before anything of this launch can end
     const unsigned int exch0 = tp ? *a.epoch * (unsigned int)a.n_layers : 0u;
-    int *ready_gu = a.state + FF_STATE_HEADER / sizeof(int), *ready_d = ready_gu + FF_READY_WORDS;
+    int *ready_gu = a.state + FF_STATE_HEADER / sizeof(int), *ready_d = ready_gu + FF_READY_WORDS * FF_READY_STRIDE;
     float *sumsq = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(a.state) + FF_STATE_HEADER + FF_READY_BYTES);
     // Per-group readiness: a down unit needs only its own 128 SwiGLU outputs, so it starts as soon as the
     // four sub-strips that produce them are finished; an SM that is done with its gate/up units does not wait for the
@@ -391,9 +393,9 @@ ffn_fused_kernel(const __grid_constant__ CUtensorMap tmXi, const __grid_constant
                     } else if (ld_acquire_gpu(p ? done_gu : done_d) >= target) {
                         phase_open = true;
                     } else if (p) {
-                        if (!wait_count(ready_gu + g, 4 * (l + 1), a.wait_limit)) return false;
+                        if (!wait_count(ready_gu + g * FF_READY_STRIDE, 4 * (l + 1), a.wait_limit)) return false;
                     } else if (l > 0) {
-                        if (!wait_count(ready_d + g, 2 * l, a.wait_limit)) return false;
+                        if (!wait_count(ready_d + g * FF_READY_STRIDE, 2 * l, a.wait_limit)) return false;
                     }  // layer 0 reads the caller's input
                     fence_proxy_async_all();  // generic-proxy writes of the previous phase before the tensor copies read them
                     return true;
@@ -494,9 +496,11 @@ ffn_fused_kernel(const __grid_constant__ CUtensorMap tmXi, const __grid_constant
                     uint32_t o[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        const float lo = bf16_bits_to_f32(f32_to_bf16_bits((bf16x2_lo(hw[e]) * rstd) * bf16x2_lo(gw[e])));
-                        const float hi = bf16_bits_to_f32(f32_to_bf16_bits((bf16x2_hi(hw[e]) * rstd) * bf16x2_hi(gw[e])));
-                        o[e] = (uint32_t)bf16_value_to_f16_bits(lo) | ((uint32_t)bf16_value_to_f16_bits(hi) << 16);
+                        // two conversions for two values each: to bf16, and of that to fp16 (one by one: 2 % of a small layer)
+                        const __nv_bfloat162 n2 = __floats2bfloat162_rn((bf16x2_lo(hw[e]) * rstd) * bf16x2_lo(gw[e]), (bf16x2_hi(hw[e]) * rstd) * bf16x2_hi(gw[e]));
+                        const uint32_t nb = *reinterpret_cast<const uint32_t *>(&n2);
+                        const __half2 h2 = __floats2half2_rn(bf16x2_lo(nb), bf16x2_hi(nb));
+                        o[e] = *reinterpret_cast<const uint32_t *>(&h2);
                     }
                     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(o[0]), "r"(o[1]), "r"(o[2]),
                                  "r"(o[3])
@@ -615,7 +619,7 @@ ffn_fused_kernel(const __grid_constant__ CUtensorMap tmXi, const __grid_constant
         if (lane == 0) {
             // this sub-strip's 32 SwiGLU outputs are a quarter of down k-group 2 v + cw / 4; its 64 hidden values are half
             // of gate/up k-group 4 v + cw / 2
-            if (fg) atomicAdd(p ? ready_d + 4 * v + cw / 2 : ready_gu + 2 * v + cw / 4, 1);
+            if (fg) atomicAdd(p ? ready_d + (4 * v + cw / 2) * FF_READY_STRIDE : ready_gu + (2 * v + cw / 4) * FF_READY_STRIDE, 1);
             atomicAdd(p ? done_d : done_gu, 1);
         }
     };
