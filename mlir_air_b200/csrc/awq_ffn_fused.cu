@@ -68,6 +68,7 @@ struct alignas(128) FusedLayer {
 };
 static_assert(sizeof(FusedLayer) % 128 == 0, "tensor maps must stay 64-byte aligned in the array");
 
+constexpr long long FF_FEW_MAX_WEIGHTS = 250000000;
 constexpr int FF_MAX_LAYERS = 1024;  // 2 claim words per layer in shared memory
 // State of one launch in the workspace, zeroed by the launcher: two phase counters; per k-group of the down
 // projection (128 SwiGLU outputs) how many of the four 32-output sub-strips that feed it have been finished so far
@@ -210,6 +211,7 @@ __device__ __forceinline__ void ff_load_residual(uint4 (&rres)[2], const uint16_
     }
 }
 
+template <bool FEW>  // one or two batch rows (sk_handover)
 __global__ void __launch_bounds__(FF_THREADS, 1)
 ffn_fused_kernel(const __grid_constant__ CUtensorMap tmXi, const __grid_constant__ CUtensorMap tmH0,
                  const __grid_constant__ CUtensorMap tmH, const FusedArgs a) {
@@ -589,8 +591,8 @@ ffn_fused_kernel(const __grid_constant__ CUtensorMap tmXi, const __grid_constant
         // a strip shared with other halves: value and progress travel in one 64-bit atomic per sum; the warp
         // whose add completes the count has the total (gate/up and down strips use separate accumulators)
         if (seg_groups != G &&
-            !sk_handover(a.accum + ((size_t)((p ? V0 : 0) + v) * SK_CONSUMER_WARPS + cw) * SK_ACC_WORDS, own, seg_groups, G, lane,
-                         a.wait_limit, a.err_flag))
+            !sk_handover<FEW>(a.accum + ((size_t)((p ? V0 : 0) + v) * SK_CONSUMER_WARPS + cw) * SK_ACC_WORDS, own, seg_groups, G, lane,
+                              b < B, a.wait_limit, a.err_flag))
             return;
         if (failed) return;
         if (!p) {
@@ -748,7 +750,9 @@ int launch_ffn_fused(const void *plan_dev, int n_layers, const uint16_t *x, uint
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(ffn_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FF_SMEM_BYTES);
+        attr_err = cudaFuncSetAttribute(ffn_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FF_SMEM_BYTES);
+        if (attr_err == cudaSuccess)
+            attr_err = cudaFuncSetAttribute(ffn_fused_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FF_SMEM_BYTES);
     });
     if (attr_err != cudaSuccess) return check_cuda(attr_err, "fused ffn: shared memory attribute");
     const size_t need = ffn_fused_workspace_bytes(n_layers);
@@ -824,7 +828,13 @@ int launch_ffn_fused(const void *plan_dev, int n_layers, const uint16_t *x, uint
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return check_cuda(cudaLaunchKernelEx(&cfg, ffn_fused_kernel, tmXi, tmH0, tmH, a), "fused ffn launch");
+    // One or two rows and not too large a layer: the hand-over of the rows that exist only.  (One row, us per layer, all rows /
+    // those that exist: 50 M weights 18.6 / 18.1, 135 M 27.3 / 25.9, 302 M 40.6 / 40.4, 705 M 72.6 / 74.9: there the end of a phase
+    // is short beside it, and the schedule that the compiler finds for this form is the slower one.  Four rows: no difference.)
+    const bool few = B <= 2 && 3ll * H * I <= FF_FEW_MAX_WEIGHTS;
+    return check_cuda(few ? cudaLaunchKernelEx(&cfg, ffn_fused_kernel<true>, tmXi, tmH0, tmH, a)
+                          : cudaLaunchKernelEx(&cfg, ffn_fused_kernel<false>, tmXi, tmH0, tmH, a),
+                      "fused ffn launch");
 }
 
 }  // namespace awq

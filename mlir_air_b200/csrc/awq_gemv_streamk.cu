@@ -46,7 +46,7 @@ size_t gemv_streamk_workspace_clear_bytes(int N) {
     return SK_WS_ACCUM + (size_t)((N + SK_STRIP - 1) / SK_STRIP) * SK_STRIP_WORDS * 8;
 }
 
-template <int EPI, bool XH>
+template <int EPI, bool XH, bool FEW>  // FEW: one or two batch rows (sk_handover)
 __global__ void __launch_bounds__(SK_THREADS, SK_CTAS_PER_SM)
 gemv_streamk_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                     const __grid_constant__ CUtensorMap tmS, const __grid_constant__ CUtensorMap tmZ,
@@ -151,8 +151,8 @@ gemv_streamk_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
         const int b = 2 * t4 + odd;
         const int n = v * SK_STRIP + colw;
         if (seg_groups != G &&
-            !sk_handover(accum + ((size_t)v * SK_CONSUMER_WARPS + warp) * SK_ACC_WORDS, own, seg_groups, G, lane, wait_limit,
-                         err_flag))
+            !sk_handover<FEW>(accum + ((size_t)v * SK_CONSUMER_WARPS + warp) * SK_ACC_WORDS, own, seg_groups, G, lane,
+                               b < B, wait_limit, err_flag))
             return;
         if (!failed) sk_epilogue<EPI>(own, residual, y_, B, N, n, b, out_f16);
         if (EPI == EPI_F32_PUSH && !failed) sk_push_signal(push, err_flag + 8, V * SK_CONSUMER_WARPS, lane);
@@ -264,12 +264,12 @@ size_t gemv_streamk_workspace_bytes(int B, int K, int N) {
     return SK_WS_XH + rows * (size_t)(K > 0 ? K : 0) * 2;
 }
 
-template <int EPI, bool XH>
-static int launch_one(const GemvArgs &a, const uint16_t *x, const uint16_t *residual, void *y, int B) {
+template <int EPI, bool XH, bool FEW>
+static int launch_rows(const GemvArgs &a, const uint16_t *x, const uint16_t *residual, void *y, int B) {
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(gemv_streamk_kernel<EPI, XH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        attr_err = cudaFuncSetAttribute(gemv_streamk_kernel<EPI, XH, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         SK_SMEM_BYTES);
     });
     if (attr_err != cudaSuccess) return check_cuda(attr_err, "stream-K gemv: shared memory attribute");
@@ -297,10 +297,15 @@ static int launch_one(const GemvArgs &a, const uint16_t *x, const uint16_t *resi
     uint8_t *ws = reinterpret_cast<uint8_t *>(a.workspace);
     int *err_flag = reinterpret_cast<int *>(ws);
     unsigned long long *accum = reinterpret_cast<unsigned long long *>(ws + SK_WS_ACCUM);
-    return check_cuda(launch_pdl(gemv_streamk_kernel<EPI, XH>, dim3(ctas), dim3(SK_THREADS), SK_SMEM_BYTES, a.stream, tmW,
+    return check_cuda(launch_pdl(gemv_streamk_kernel<EPI, XH, FEW>, dim3(ctas), dim3(SK_THREADS), SK_SMEM_BYTES, a.stream, tmW,
                                  tmX, tmS, tmZ, residual, y, B, a.N, G, V, a.out_format == ACT_F16 ? 1 : 0, accum, err_flag,
                                  a.push ? *a.push : PeerPush{}, wait_limit_cycles()),
                       "stream-K gemv launch");
+}
+
+template <int EPI, bool XH>
+static int launch_one(const GemvArgs &a, const uint16_t *x, const uint16_t *residual, void *y, int B) {
+    return B <= 2 ? launch_rows<EPI, XH, true>(a, x, residual, y, B) : launch_rows<EPI, XH, false>(a, x, residual, y, B);
 }
 
 template <bool XH>

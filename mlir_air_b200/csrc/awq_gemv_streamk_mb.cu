@@ -175,8 +175,8 @@ gemv_streamk_mb_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
             sk_lane_exchange(res[t], odd, own);
             const int b = 8 * t + 2 * t4 + odd;
             if (seg_groups != G &&
-                !sk_handover(accum + ((size_t)(v * T + t) * SK_CONSUMER_WARPS + warp) * SK_ACC_WORDS, own, seg_groups, G, lane,
-                             wait_limit, err_flag))
+                !sk_handover<false>(accum + ((size_t)(v * T + t) * SK_CONSUMER_WARPS + warp) * SK_ACC_WORDS, own, seg_groups, G, lane,
+                             true, wait_limit, err_flag))
                 continue;
             if (!failed) sk_epilogue<EPI>(own, residual, y_, B, N, n, b, out_f16);
         }

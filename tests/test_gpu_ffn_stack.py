@@ -399,3 +399,20 @@ def test_gemm_decode_rejects_what_it_cannot_run(ops):
     ws8 = ops.GemmDecodeWorkspace(256, batch=64, K=256)
     with pytest.raises(AwqBackendError):  # and takes 32 rows at most
         ops.gemm_decode(to_dev(randn_bf16((33, 256), seed=1)), w, ws8, f8=True)
+
+
+@pytest.mark.parametrize("B", [1, 2, 3, 8])
+def test_hand_over_of_used_rows_leaves_the_words_zero(ops, B):
+    """One and two rows hand over only their own sums: batches of every size in turn on one workspace, and the GEMV on it, must each
+    find the accumulator words zero."""
+    from gpu_util import dev_weight, randn_bf16, synth_awq, to_dev, to_host
+    H, I = 1024, 2816
+    layers_np = _layers_np(H, I, 1, seed=5)
+    plan, gus, downs, gammas = _plan(ops, layers_np)
+    ws = ops.Workspace(max(H, I), 2 * I)
+    w = synth_awq(H, 1536, 128, seed=9)
+    for b in (B, 8, B, 1, B):
+        x = randn_bf16((b, H), seed=b)
+        assert O.rel_l2(to_host(ops.ffn_stack_decode(plan, to_dev(x), ws)), _oracle_stack(x, layers_np)) <= REL_L2_TOL
+        assert O.rel_l2(to_host(ops.gemv(to_dev(x), dev_weight(*w), ws)), O.gemv_A_ref(x, *w, 128)) <= REL_L2_TOL
+    ws.check()
