@@ -220,8 +220,8 @@ rmsnorm_split_kernel(const uint16_t *__restrict__ h, const uint16_t *__restrict_
     __shared__ float red[RS_THREADS / 32];
     pdl_launch_dependents();
     const int m = blockIdx.x, lane = threadIdx.x & 31, n_chunks = K >> 3, mine = blockIdx.y * RS_THREADS + threadIdx.x;
-    const uint4 gt = mine < n_chunks ? *reinterpret_cast<const uint4 *>(gamma + 8 * mine) : make_uint4(0u, 0u, 0u, 0u);
     pdl_wait();
+    const uint4 gt = mine < n_chunks ? *reinterpret_cast<const uint4 *>(gamma + 8 * mine) : make_uint4(0u, 0u, 0u, 0u);
     uint4 t[RS_CHUNKS];
     float ss = 0.f;
 #pragma unroll

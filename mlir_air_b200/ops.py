@@ -17,7 +17,8 @@ def _ptr(t: Optional[torch.Tensor]):
 
 # torch.cuda.current_stream().cuda_stream without the Stream object in between (3.1 -> 0.2 us, of about 13 for an operator call
 # whose kernel takes 3); the operators' tensors exist, so CUDA is initialised
-_raw_stream, _device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # (a torch built without CUDA can import this module)
+_device = getattr(torch._C, "_cuda_getDevice", None)
 
 
 def _stream():
