@@ -22,7 +22,7 @@
 //   work     token rows are counted in units of 32 and the (column tile, token unit) plane is cut into one contiguous
 //            range per pair, so that no pair idles in a partial last wave whatever M and N are; a range is walked in
 //            pieces of nearly equal width inside a column tile.  Where the cuts may lie is chosen on the host by a cost
-//            model (pair_cost below)
+//            model (awq_pair_plan.cuh)
 //   TMEM     int4: accumulators at 0 (two sets of 192 columns, or one of 256), four weight buffers of 32 columns (64 k)
 //            from 384 on; bf16: two accumulator sets of 256
 //   epilogue accumulators -> bf16 (or f32 + residual -> bf16) -> stmatrix.trans into a staging tile in shared memory ->
@@ -35,6 +35,7 @@
 #include <mutex>
 
 #include "awq_common.cuh"
+#include "awq_pair_plan.cuh"
 #include "awq_ptx.cuh"
 #include "awq_tcgen05.cuh"
 
@@ -43,8 +44,7 @@ namespace awq {
 int encode_tensor_map_2d(CUtensorMap *map, int dtype, const void *base, uint64_t dim0, uint64_t dim1,
                          uint64_t stride1_bytes, uint32_t box0, uint32_t box1, int swizzle);
 
-constexpr int GP_BN = 256, GP_HALF = 128, GP_BK = 64, GP_GROUP = 128;
-constexpr int GP_UNIT = 32, GP_MAX_UNITS = 8;              // token rows: unit of the schedule, most units per piece
+constexpr int GP_HALF = 128, GP_GROUP = 128;
 constexpr int GP_X_UNIT_BYTES = GP_UNIT / 2 * GP_BK * 2;   // 2 KB: this CTA's half of a unit of token rows x 64 k
 constexpr int GP_EPI_WARPS = 8;
 constexpr int GP_STAGING_STRIDE = GP_HALF * 2 + 16;        // bytes of a token row in the staging tile (+16: no bank conflicts)
@@ -90,57 +90,6 @@ constexpr uint32_t GP_IDESC_BASE = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32
 struct PairMaps {
     CUtensorMap x[GP_MAX_UNITS];  // token rows: box of 16 (i + 1) rows x 64 k
     CUtensorMap w, s, z;
-};
-
-// The schedule of a launch.  Token rows are counted in units of 32, R of them per column tile.  First `waves` rounds in
-// which the P pairs take neighbouring tiles of the (column tile, token tile) grid, token tiles innermost (N_T nearly equal
-// ones per column tile): the pairs of a round share token rows and weights in L2.  What does not fill a round is cut
-// evenly: units from `base` on, counted column tile by column tile, one contiguous range per pair, where a cut closer than
-// `snap` units to a column tile's edge moves there.
-// With S > 1, P pairs share the plane S times: the pairs of part s multiply the s-th part of K and leave f32 sums, which a
-// second kernel adds up (gemm_pair_sum_kernel).
-struct PairPlan {
-    int P, R, C, max_units, sets, waves, NT, base, snap, S;
-    __host__ __device__ int cut(int p) const {
-        const int v = base + (int)((long long)p * ((long long)R * C - base) / P), r = v % R;
-        if (r == 0) return v;
-        if (r <= snap) return v - r > base ? v - r : base;
-        return R - r <= snap ? v + R - r : v;
-    }
-};
-
-struct PairWalk {
-    const PairPlan &pl;
-    int p, w = 0, cur, end, seg_tile = 0, seg_a = 0, seg_len = 0, n = 0, i = 0;
-    int tile = 0, unit = 0, units = 0;  // the current piece
-    __host__ __device__ PairWalk(int p_, const PairPlan &plan) : pl(plan), p(p_), cur(plan.cut(p_)), end(plan.cut(p_ + 1)) {}
-    __host__ __device__ bool next() {
-        int a, b;
-        if (w < pl.waves) {
-            const int t = w * pl.P + p, j = t % pl.NT;
-            ++w;
-            tile = t / pl.NT;
-            a = j * pl.R / pl.NT;
-            b = (j + 1) * pl.R / pl.NT;
-        } else {
-            if (i == n) {
-                if (cur >= end) return false;
-                seg_tile = cur / pl.R;
-                seg_a = cur - seg_tile * pl.R;
-                seg_len = pl.R - seg_a < end - cur ? pl.R - seg_a : end - cur;
-                n = (seg_len + pl.max_units - 1) / pl.max_units;
-                i = 0;
-                cur += seg_len;
-            }
-            tile = seg_tile;
-            a = seg_a + i * seg_len / n;
-            b = seg_a + (i + 1) * seg_len / n;
-            ++i;
-        }
-        unit = a;
-        units = b - a;
-        return true;
-    }
 };
 
 __device__ int g_gemm_pair_error;  // 0 = ok; set when a bounded wait gave up
@@ -637,7 +586,6 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, uint16_t *__restrict__ C
 
 // Second pass of a product whose K was cut into S parts: four columns of a token row a thread, the parts' sums in their order, then
 // the epilogue (the rounding points of the kernel above).
-constexpr int GP_MAX_PARTS = 8;
 __global__ void __launch_bounds__(256)
 gemm_pair_sum_kernel(const float *__restrict__ parts, int S, uint16_t *__restrict__ C, const uint16_t *__restrict__ R, int epi, int M, int N,
                      int n_pad) {
@@ -674,35 +622,6 @@ gemm_pair_sum_kernel(const float *__restrict__ parts, int S, uint16_t *__restric
 }
 
 // ---------------------------------------------------------------------------------------------
-// The longest pair's time for a plan, in cycles.  Measured with clock64 per k-block of 64: 69 cycles per unit of 32 token
-// rows (64 at the tensor pipe's peak), but not less than about 370 with int4 weights (the chain of a dequant group: fetch
-// 240, arithmetic 630, tensor-memory store 200, over four groups) and 280 plus 35 per unit with bf16 ones (its bytes at the
-// 59 bytes per cycle and SM that L2 delivers: a narrow piece's stage is mostly weights).  A piece's drain is exposed where there is one accumulator set: 2,600 cycles.  Parts of K: their sums
-// cross L2 twice, and the second pass is a launch.
-static size_t pair_parts_bytes(int M, int N, int S) { return (size_t)S * M * ((N + GP_BN - 1) / GP_BN * GP_BN) * 4; }
-constexpr size_t GP_PARTS_MAX_BYTES = 64u << 20;  // about half of L2
-static long long pair_cost(const PairPlan &pl, int KB_all, bool w4, int M) {
-    const int KB = (KB_all / 2 + pl.S - 1) / pl.S * 2;
-    const int floor_cycles = w4 ? 370 : 280, floor_unit = w4 ? 0 : 35, drain = pl.sets == 2 ? 600 : 3000;
-    auto segment = [&](int len, int n) -> long long {  // `len` units of one column tile in n pieces
-        const long long least = (long long)n * floor_cycles + (long long)len * floor_unit;
-        const long long kblock = 69 * len > least ? 69 * len : least;
-        return KB * kblock + (long long)n * drain;
-    };
-    auto cut_up = [&](int len) -> long long { return len <= 0 ? 0 : segment(len, (len + pl.max_units - 1) / pl.max_units); };
-    const long long whole = cut_up(pl.R);
-    long long worst = 0;
-    int a = pl.cut(0);
-    for (int p = 0; p < pl.P && a < pl.R * pl.C; ++p) {
-        const int b = pl.cut(p + 1), ta = a / pl.R, tb = b / pl.R;
-        const long long t = ta == tb ? cut_up(b - a) : cut_up((ta + 1) * pl.R - a) + (tb - ta - 1) * whole + cut_up(b - tb * pl.R);
-        if (t > worst) worst = t;
-        a = b;
-    }
-    const long long parts = pl.S > 1 ? 6000 + (long long)pl.S * M * pl.C * GP_BN * 4 / 1000 : 0;
-    return worst + pl.waves * segment((pl.R + pl.NT - 1) / pl.NT, 1) + parts;
-}
-
 // The cheapest plan for a shape: a pure function of the sizes; the last shapes are remembered, the search takes microseconds.
 template <bool W4>
 static PairPlan pair_plan(int M, int N, int K, int all_pairs, bool may_split) {
@@ -712,54 +631,11 @@ static PairPlan pair_plan(int M, int N, int K, int all_pairs, bool may_split) {
     };
     thread_local Memo memo[64];
     Memo &m = memo[(((unsigned)M * 2654435761u ^ (unsigned)N * 2246822519u ^ (unsigned)K * 3266489917u) >> 27) * 2 + may_split];
-    if (m.M == M && m.N == N && m.K == K && m.pairs == all_pairs && m.split == may_split) return m.plan;
-    PairPlan pl, best_plan;
-    pl.R = (M + GP_UNIT - 1) / GP_UNIT;
-    pl.C = (N + GP_BN - 1) / GP_BN;
-    const int KB = (K + 2 * GP_BK - 1) / (2 * GP_BK) * 2;
-    long long best = -1;
-    auto consider = [&] {
-        const long long c = pair_cost(pl, KB, W4, M);
-        if (best < 0 || c < best) best = c, best_plan = pl;
-    };
-    const int nt_min = (pl.R + GP_MAX_UNITS - 1) / GP_MAX_UNITS;
-    // parts of K: of eight k-blocks at least, and not where the plane alone gives every pair two pieces
-    for (pl.S = 1; pl.S == 1 || (may_split && pl.S <= GP_MAX_PARTS && KB >= 8 * pl.S && pl.C * nt_min < 2 * all_pairs &&
-                                 pair_parts_bytes(M, N, pl.S) <= GP_PARTS_MAX_BYTES);
-         pl.S += pl.S < 4 ? 1 : 2) {
-        const int pairs = all_pairs / pl.S;
-        for (pl.NT = nt_min; pl.NT <= pl.R && pl.NT < nt_min + 4; ++pl.NT) {
-            const int tiles = pl.NT * pl.C;
-            pl.max_units = (pl.R + pl.NT - 1) / pl.NT;  // of a tile, and of a piece of what is cut evenly
-            pl.sets = !W4 || pl.max_units <= GP_MAX_UNITS / 2 ? 2 : 1;
-            pl.P = tiles < pairs ? tiles : pairs;
-            for (int back = 0; back < 2 && back <= tiles / pl.P; ++back) {  // rounds; the rest is cut evenly
-                pl.waves = tiles / pl.P - back;
-                const int t = pl.waves * pl.P;
-                pl.base = t / pl.NT * pl.R + t % pl.NT * pl.R / pl.NT;
-                if (t == tiles) {
-                    pl.snap = 0;
-                    consider();
-                    continue;
-                }
-                if (pl.S > 1) continue;  // parts of whole tiles only (512 x 8192 x 2048 bf16: 20.8 us so, 23.1 in three parts cut evenly)
-                for (int sn : {0, 2, pl.R}) {
-                    pl.snap = sn;
-                    consider();
-                }
-            }
-            if (pl.S == 1 && tiles < pairs && pl.R * pl.C > tiles) {  // fewer tiles than pairs: cut everything evenly over all pairs
-                pl.P = pl.R * pl.C < pairs ? pl.R * pl.C : pairs;
-                pl.waves = pl.base = 0;
-                for (int sn : {0, 2}) {
-                    pl.snap = sn;
-                    consider();
-                }
-            }
-        }
+    if (m.M != M || m.N != N || m.K != K || m.pairs != all_pairs || m.split != may_split) {
+        m.plan = pair_search(W4, M, N, K, all_pairs, may_split);
+        m.M = M, m.N = N, m.K = K, m.pairs = all_pairs, m.split = may_split;
     }
-    m.M = M, m.N = N, m.K = K, m.pairs = all_pairs, m.split = may_split, m.plan = best_plan;
-    return best_plan;
+    return m.plan;
 }
 
 static int pair_count() {
