@@ -466,6 +466,8 @@ def ffn_layer_decode(x, w_gateup: AwqWeight, w_down: AwqWeight, ws: GemmDecodeWo
     B, H, I = x.shape[0], w_gateup.K, w_gateup.N // 2
     if w_down.K != I or w_down.N != H:
         raise _lib.AwqBackendError(f"down weight must be [{I}, {H}], got [{w_down.K}, {w_down.N}]")
+    if w_down.group_size != w_gateup.group_size:
+        raise _lib.AwqBackendError(f"both weights must have one group size, got {w_gateup.group_size} and {w_down.group_size}")
     if out is None:
         out = torch.empty((B, H), dtype=torch.bfloat16, device=x.device)
     _lib.call("awq_b200_ffn_layer_decode_bf16", _ptr(x), _ptr(_want(gamma, torch.bfloat16, "gamma")), float(eps), _ptr(w_gateup.qweight),
