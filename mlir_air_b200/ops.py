@@ -468,8 +468,12 @@ def ffn_layer_decode(x, w_gateup: AwqWeight, w_down: AwqWeight, ws: GemmDecodeWo
         raise _lib.AwqBackendError(f"down weight must be [{I}, {H}], got [{w_down.K}, {w_down.N}]")
     if w_down.group_size != w_gateup.group_size:
         raise _lib.AwqBackendError(f"both weights must have one group size, got {w_gateup.group_size} and {w_down.group_size}")
+    if gamma.numel() != H:
+        raise _lib.AwqBackendError(f"gamma must have {H} elements, got {gamma.numel()}")
     if out is None:
         out = torch.empty((B, H), dtype=torch.bfloat16, device=x.device)
+    if tuple(out.shape) != (B, H) and not (B == 1 and tuple(out.shape) == (H,)):
+        raise _lib.AwqBackendError(f"out must be [{B}, {H}], got {tuple(out.shape)}")
     _lib.call("awq_b200_ffn_layer_decode_bf16", _ptr(x), _ptr(_want(gamma, torch.bfloat16, "gamma")), float(eps), _ptr(w_gateup.qweight),
               _ptr(w_gateup.qzeros), _ptr(w_gateup.scales), _ptr(w_down.qweight), _ptr(w_down.qzeros), _ptr(w_down.scales),
               _ptr(_want(out, torch.bfloat16, "out")), B, H, I, w_gateup.group_size, _ptr(ws.buf), ws.nbytes, _stream())

@@ -41,3 +41,22 @@ def test_refuses_weights_of_different_group_sizes(launched, gu_gs, down_gs):
     with pytest.raises(_lib.AwqBackendError, match="group size"):
         _call(gu_gs=gu_gs, down_gs=down_gs)
     assert not launched
+
+
+@pytest.mark.parametrize("gamma", [H - 128, 2 * H, (2, H)])
+def test_refuses_a_norm_weight_of_another_length(launched, gamma):
+    with pytest.raises(_lib.AwqBackendError, match="gamma"):
+        _call(gamma=gamma)
+    assert not launched
+
+
+@pytest.mark.parametrize("x,out", [((9, H), (8, H)), ((9, H), (9, I)), ((9, H), (H, 9)), ((H,), (2, H))])
+def test_refuses_an_output_of_another_shape(launched, x, out):
+    with pytest.raises(_lib.AwqBackendError, match="out"):
+        _call(x=x, out=out)
+    assert not launched
+
+
+def test_one_row_may_be_a_vector(launched):
+    assert _call(x=(H,)).shape == (1, H) and _call(x=(H,), out=(H,)).shape == (H,) and _call(x=(1, H), out=(1, H)).shape == (1, H)
+    assert len(launched) == 3
