@@ -119,13 +119,17 @@ class DecodeFFNStack:
     kernels of the ranks wait for one another with a limit of about a second, so a one-element
     allreduce is enqueued in front of each launch (also inside the captured graph); it makes the
     ranks' kernels start together however far apart the host threads are.
+    `one_call`: on one GPU a layer of 9 to 64 rows is one call of ops.ffn_layer_decode where that takes
+    it; False: the norm and the two products as calls of their own.
     """
 
     def __init__(self, layers: Sequence[FFNLayer], hidden: int, max_batch: int = 64, eps: float = 1e-5,
-                 group=None, device="cuda", fused: bool = True, peer_push: bool = False, align_ranks: bool = True):
+                 group=None, device="cuda", fused: bool = True, peer_push: bool = False, align_ranks: bool = True,
+                 one_call: bool = True):
         self.layers = list(layers)
         self.hidden = hidden
         self.eps = eps
+        self.one_call = one_call
         self.group = group
         self.device = torch.device(device)
         self.tp = 1 if group is None else torch.distributed.get_world_size(group)
@@ -201,17 +205,20 @@ class DecodeFFNStack:
     def uses_fused(self, batch: int) -> bool:
         return self.plan is not None and batch <= 8
 
-    # From this batch on one GPU, a layer is two batched-decode tensor-core GEMMs (weights streamed once
-    # per layer whatever the batch, SwiGLU / residual in the epilogue) instead of one GEMV pass per 8 rows
-    # (9-16 rows: the same time as the two-tile GEMV pass at the 70B dimensions, 9 % less at the 7B ones).
+    # From this batch on, a layer runs on the batched-decode tensor-core GEMMs (weights streamed once per layer whatever the
+    # batch, SwiGLU / residual in the epilogue) instead of one GEMV pass per 8 rows (9-16 rows: the same time as the two-tile
+    # GEMV pass at the 70B dimensions, 9 % less at the 7B ones).
     GEMM_BATCH = 9
-    # Up to here the GEMM is the kernel that feeds the tensor core the packed nibbles and split token rows as fp8 (scale and
-    # zero point in f32): 10 % faster than the 16-bit-operand kernel at 16 rows, 3 % at 32, and no weight is rounded.
+    # Where the two products are calls of their own (tensor-parallel ranks; one GPU: `one_call` off, or a layer that
+    # ops.ffn_layer_decode does not take), up to here they may run on the kernel that feeds the tensor core the packed nibbles
+    # and split token rows as fp8 (scale and zero point in f32): 10 % faster than the 16-bit-operand kernel at 16 rows, 3 % at
+    # 32, and no weight is rounded.
     GEMM_F8_BATCH = 32
     # ... where a layer is large enough for its three launches per product to pay: measured on one box (us per layer,
     # 16-bit against fp8 operands, by weights per layer on this rank): 35 M 21.0 / 22.3 at 16 rows and 24.0 / 27.0 at 32;
     # 88 M 28.6 / 30.9 at 32; 135 M 33.4 / 32.6 and 36.6 / 38.3; 176 M 38.2 / 36.0 and 40.4 / 41.2; 352 M 60.3 / 54.7 and
-    # 63.4 / 59.9; 705 M 104.4 / 89.6 and 111.3 / 99.4.
+    # 63.4 / 59.9; 705 M 104.4 / 89.6 and 111.3 / 99.4.  A stack that is given other bars than these chooses between the separate
+    # products by them on one GPU too.
     GEMM_F8_MIN_WEIGHTS = {16: 120e6, 32: 250e6}
 
     def uses_gemm_f8(self, batch: int) -> bool:
@@ -223,9 +230,8 @@ class DecodeFFNStack:
         return all(self.gemm_ws.fits_f8(batch, w.K, w.N) for l in self.layers for w in (l.gateup, l.down))
 
     def uses_layer(self, batch: int) -> bool:
-        """One GPU: each layer is one call (fp8-operand kernel up to 32 rows, 16-bit one beyond).  A stack that was given GEMM_F8_MIN_WEIGHTS of its own runs
-        the separate products that this chooses between."""
-        if self.tp > 1 or "GEMM_F8_MIN_WEIGHTS" in self.__dict__ or not self.uses_gemm(batch):
+        """One GPU: each layer is one call (fp8-operand kernel up to 32 rows, 16-bit one beyond)."""
+        if self.tp > 1 or not self.one_call or self.GEMM_F8_MIN_WEIGHTS != DecodeFFNStack.GEMM_F8_MIN_WEIGHTS or not self.uses_gemm(batch):
             return False
         fits = getattr(self.gemm_ws, "fits_layer", None)
         return fits is not None and all(

@@ -60,3 +60,25 @@ def test_refuses_an_output_of_another_shape(launched, x, out):
 def test_one_row_may_be_a_vector(launched):
     assert _call(x=(H,)).shape == (1, H) and _call(x=(H,), out=(H,)).shape == (H,) and _call(x=(1, H), out=(1, H)).shape == (1, H)
     assert len(launched) == 3
+
+
+def _stack(**attributes):
+    from types import SimpleNamespace as NS
+    from mlir_air_b200 import ffn
+    w = lambda K, N: NS(K=K, N=N, group_size=128)
+    st = object.__new__(ffn.DecodeFFNStack)  # (the constructor's buffers need a GPU; the choice of the path does not)
+    layer = NS(gateup=w(H, 2 * I), down=w(I, H), gamma=torch.ones(H))
+    st.__dict__.update(tp=1, plan=None, one_call=True, layers=[layer] * 3, gemm_ws=ops.GemmDecodeWorkspace(2 * I, device="cpu", K=I), **attributes)
+    return st
+
+
+def test_one_call_layers_are_switched_by_their_argument():
+    from mlir_air_b200.ffn import DecodeFFNStack
+    st = _stack()
+    assert [st.uses_layer(b) for b in (8, 9, 32, 33, 64, 65)] == [False, True, True, True, True, False] and st.launches_per_step(16) == 15
+    st.one_call = False
+    assert not any(st.uses_layer(b) for b in range(1, 66)) and st.uses_gemm(16) and st.launches_per_step(16) == 15 and not st.uses_gemm_f8(16)
+    # the class's own size bars, given to a stack again, change nothing; others choose between the separate products
+    assert _stack(GEMM_F8_MIN_WEIGHTS=dict(DecodeFFNStack.GEMM_F8_MIN_WEIGHTS)).uses_layer(16)
+    st = _stack(GEMM_F8_MIN_WEIGHTS={16: 0, 32: 0})
+    assert not st.uses_layer(16) and st.uses_gemm_f8(16) and st.launches_per_step(16) == 21 and st.launches_per_step(33) == 15

@@ -56,3 +56,33 @@ def test_layer_refuses():
         ops.ffn_layer_decode(torch.zeros((65, 128), dtype=torch.bfloat16, device="cuda"), w, d, ws, g)
     with pytest.raises(AwqBackendError):
         ops.ffn_layer_decode(torch.zeros((8, 128), dtype=torch.bfloat16, device="cuda"), w, w, ws, g)
+
+
+@pytest.mark.parametrize("B", [9, 16, 33, 64])
+def test_stack_in_one_call_per_layer(B):
+    """What a stack on one GPU runs by itself, in its three call forms, and the separate products that `one_call` = False asks for."""
+    import torch
+    from gpu_util import dev_weight, randn_bf16, synth_awq, to_dev, to_host
+    from mlir_air_b200 import ffn, ops
+    H, I, L = 512, 1408, 3
+    layers_np = []
+    for l in range(L):
+        gate, up = synth_awq(H, I, 128, seed=10 * l), synth_awq(H, I, 128, seed=10 * l + 1)
+        down = synth_awq(I, H, 128, seed=10 * l + 2, scale_lo=0.0005, scale_hi=0.004)
+        layers_np.append((gate, up, down, (np.random.default_rng(l).standard_normal(H) * 0.1 + 1.0).astype(bfloat16)))
+    layers = [ffn.FFNLayer(ops.interleave_gate_up(dev_weight(*g), dev_weight(*u)), dev_weight(*d), to_dev(gm)) for g, u, d, gm in layers_np]
+    x = randn_bf16((B, H), seed=B)
+    ref = x
+    for gate, up, down, gamma in layers_np:
+        ref = O.ffn_layer_A_ref(ref, gamma, gate, up, down, 128)
+    stack = ffn.DecodeFFNStack(layers, H)
+    assert stack.uses_layer(B) and stack.launches_per_step(B) == 5 * L
+    y = stack.step(to_dev(x))
+    stack.load_input(to_dev(x))
+    assert torch.equal(stack.replay(B), y)
+    assert np.array_equal(stack.forward_host(x).view(np.uint16), to_host(y).view(np.uint16))
+    assert O.rel_l2(to_host(y), ref) <= L * REL_L2_TOL
+    apart = ffn.DecodeFFNStack(layers, H, one_call=False)
+    assert not apart.uses_layer(B) and apart.uses_gemm(B)
+    assert O.rel_l2(to_host(apart.step(to_dev(x))), ref) <= L * REL_L2_TOL
+    stack.check(), apart.check()
