@@ -362,9 +362,9 @@ int awq_b200_gemm_decode_act(const void *A, int a_format, const int32_t *qweight
 
 /* The same product for M <= 32 token rows with the packed nibbles themselves as the tensor core's operand
  * (a nibble q in a byte is the e4m3 number q * 2^-9) and the token rows split into two e4m3 pieces per
- * element (exact for a value of 8 significant bits, i.e. any bf16 value or an fp16 copy of one, within
- * 2^-14 of its row's largest magnitude; a genuine fp16 value is rounded to 8 significant bits, as a bf16
- * conversion would); zero point and scale are
+ * element (exact for a value of 8 significant bits, i.e. any bf16 value or an fp16 copy of one, from 2^-13 of
+ * its row's largest magnitude on; a smaller one keeps an absolute error of at most 2^-21 of that magnitude;
+ * a genuine fp16 value is rounded to 8 significant bits, as a bf16 conversion would); zero point and scale are
  * applied to the per-group sums in f32, as the reference's golden does, so no weight is rounded.  Three
  * launches: the split of the token rows, the product, the addition of the partial sums.  Arguments as
  * awq_b200_gemm_decode_act; the workspace also holds the split rows, hence K in its size. */
@@ -375,7 +375,9 @@ int awq_b200_gemm_decode_f8(const void *A, int a_format, const int32_t *qweight,
                             size_t workspace_bytes, awq_stream_t stream);
 
 /* y [B, N] = x [B, K] @ W (+ residual), as awq_b200_gemv_bf16 / awq_b200_gemv_f32 (y_f32 != 0) give it, for 9 <= B <= 64 bf16 rows, on
- * the fp8-operand kernel in passes of up to 32 rows.  No value is out of range (an infinity or a NaN shows in the output).
+ * the fp8-operand kernel in passes of up to 32 rows.  No value is out of range (an infinity or a NaN shows in the output).  A row is
+ * split as awq_b200_gemm_decode_f8 splits it, but per quantisation group: exact from 2^-13 of the largest magnitude that the row
+ * has in the group on, smaller elements to 2^-21 of that magnitude.  No weight is rounded.
  * awq_b200_gemv_rows_workspace_bytes: scratch, 0 where this does not apply or another kernel was asked for
  * (awq_b200_set_decode_kernel).  The workspace needs no initialisation; calls that share one must not overlap. */
 size_t awq_b200_gemv_rows_workspace_bytes(int B, int K, int N, int group_size);
@@ -387,7 +389,8 @@ int awq_b200_gemv_rows_bf16(const uint16_t *x, const int32_t *qweight, const int
 /* One decode FFN layer for 1 <= M <= 64 token rows on the batched-decode GEMMs (up to 32 rows the one with fp8 operands):
  *     out [M, H] = bf16(x + down(swiglu(gateup . rmsnorm(x, gamma))))
  * gate/up column-interleaved [H, 2I], group 128, H and I multiples of 128, H <= 16384; out may be x.  Five launches: the
- * norm and the SwiGLU are written in the form that the next product reads.  The workspace needs no initialisation
+ * norm and the SwiGLU are written in the form that the next product reads: up to 32 rows split as awq_b200_gemv_rows_bf16 splits
+ * them (with its bounds), beyond as fp16, the weights then rounded to fp16 too.  The workspace needs no initialisation
  * and may be shared with awq_b200_gemm_decode_*. */
 size_t awq_b200_ffn_layer_decode_workspace_bytes(int M, int H, int I);
 int awq_b200_ffn_layer_decode_bf16(const uint16_t *x, const uint16_t *gamma, float eps,

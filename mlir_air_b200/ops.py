@@ -169,7 +169,9 @@ GEMV_ROWS_MIN_WEIGHTS = {16: 100e6, 64: 32e6}
 
 def gemv(x, w: AwqWeight, ws: Workspace, residual=None, out=None, f32_out=False, x_f16=False):
     """y [B, N] = x [B, K] @ W (+ residual); bf16 with one rounding, or the f32 partial.
-    x is bf16, or fp16 (the library's internal activation format) with x_f16."""
+    x is bf16, or fp16 (the library's internal activation format) with x_f16.  bf16 rows are multiplied as they are or as
+    fp16; more than 8 rows on large weights (GEMV_ROWS_MIN_WEIGHTS) as two fp8 pieces, exact for an element from 2^-13 of the
+    largest magnitude in its row's quantisation group on, smaller ones to 2^-21 of that magnitude."""
     x = _x2d(x, w.K, x_f16)
     B = x.shape[0]
     if out is None:
@@ -461,7 +463,8 @@ def gemm_decode(A, w: AwqWeight, ws: GemmDecodeWorkspace, out=None, residual=Non
 
 def ffn_layer_decode(x, w_gateup: AwqWeight, w_down: AwqWeight, ws: GemmDecodeWorkspace, gamma, eps=1e-5, out=None):
     """out [B, H] = bf16(x + down(swiglu(gateup . rmsnorm(x, gamma)))) for a decode batch of up to 64 rows: one call, five
-    launches (norm, product, SwiGLU, product, residual add)."""
+    launches (norm, product, SwiGLU, product, residual add).  Between the kernels the bf16 values of up to 32 rows are two fp8
+    pieces each (bounds as in `gemv`) and no weight is rounded; more rows are fp16, and so are the weights."""
     x = _x2d(x, w_gateup.K)
     B, H, I = x.shape[0], w_gateup.K, w_gateup.N // 2
     if w_down.K != I or w_down.N != H:

@@ -44,6 +44,32 @@ def test_layer_vs_oracle(B, H, I):
     assert O.rel_l2(d[:, small], r[:, small]) <= 1e-2
 
 
+@pytest.mark.parametrize("B", [9, 32])
+def test_large_normalised_values_beside_small_ones(B):
+    """A norm weight of 300 in every group, whose gate/up weights are at their zero points, so that gate and up are sums of the
+    other values, which the split keeps to 2^-21 of the large one: nothing beside their bf16 rounding.  Judged column by column."""
+    from gpu_util import dev_weight, randn_bf16, synth_awq, to_dev, to_host
+    from mlir_air_b200 import ops
+    H, I = 512, 1408
+    def at_zero(w):
+        qw, qz, s = w
+        nibs = O.unpack_awq_int32(qw)
+        nibs[5::128] = O.unpack_awq_int32(qz)
+        return O.pack_awq_int32(nibs), qz, s
+    gate, up = at_zero(synth_awq(H, I, 128, seed=1)), at_zero(synth_awq(H, I, 128, seed=2))
+    down = synth_awq(I, H, 128, seed=3, scale_lo=0.0005, scale_hi=0.004)
+    gamma = (np.random.default_rng(4).standard_normal(H) * 0.1 + 1.0).astype(bfloat16)
+    gamma[5::128] = 300.0
+    x = (np.asarray(randn_bf16((B, H), seed=B), dtype=np.float32) * 2.0 ** -10).astype(bfloat16)  # (the residual does not hide the layer)
+    ws = ops.GemmDecodeWorkspace(2 * I, batch=64, K=I)
+    y = to_host(ops.ffn_layer_decode(to_dev(x), ops.interleave_gate_up(dev_weight(*gate), dev_weight(*up)), dev_weight(*down), ws,
+                                     to_dev(gamma))).astype(np.float64)
+    ops.gemm_check()
+    ref = O.ffn_layer_A_ref(x, gamma, gate, up, down, 128).astype(np.float64)
+    # the rounding points that REL_L2_TOL counts; a column has only B values: twice as much
+    assert (np.linalg.norm(y - ref, axis=0) <= 2 * REL_L2_TOL * np.linalg.norm(ref, axis=0)).all()
+
+
 def test_layer_refuses():
     import torch
     from gpu_util import dev_weight, synth_awq

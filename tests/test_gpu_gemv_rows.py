@@ -39,6 +39,37 @@ def test_vs_oracle(B, K, N, monkeypatch):
     ws.check()
 
 
+@pytest.mark.parametrize("B,big,small", [(16, 1000.0, 0.05), (33, 1000.0, 0.05), (64, 1000.0, 1.0), (32, 40.0, 0.05)])
+def test_what_the_split_keeps_of_small_values(B, big, small, monkeypatch):
+    """One large value in every group, whose weights are at their zero points: each column is the sum of the small values alone,
+    which are below 2^-13 of the large one in part, and there rounded to multiples of 2^-13 (with the large one in [128, 256))."""
+    from gpu_util import dev_weight, synth_awq, to_dev
+    from mlir_air_b200 import ops
+    monkeypatch.setattr(ops, "GEMV_ROWS_MIN_WEIGHTS", {16: 0, 64: 0})
+    K, N = 2048, 512
+    _, qz, s = synth_awq(K, N, 128, seed=11)
+    rng = np.random.default_rng(B)
+    nibs = rng.integers(0, 16, size=(K, N), dtype=np.uint8)
+    z = O.unpack_awq_int32(qz)
+    nibs[5::128] = z
+    qw = O.pack_awq_int32(nibs)
+    W = (nibs.astype(np.float64) - np.repeat(z, 128, 0)) * np.repeat(s.astype(np.float64), 128, 0)
+    x = rng.standard_normal((B, K)) * small
+    x[:, 5::128] = big
+    x = x.astype(bfloat16)
+    w, ws = dev_weight(qw, qz, s), ops.Workspace(K, N)
+    y = ops.gemv(to_dev(x), w, ws, f32_out=True).cpu().numpy().astype(np.float64)
+    ws.check()
+    err = np.linalg.norm(y - x.astype(np.float64) @ W, axis=0)
+    quantum = 2.0 ** (np.floor(np.log2(big)) - 7 - 13)
+    # elements off by up to half a quantum, independent and uniform: quantum / sqrt(12) each, times the weights' 2-norm; 1.5 for
+    # the spread over a column's rows.  And in f32 a group's two terms of 15 times the large one, which cancel: half a unit
+    # in the last place (2^-24) for each of the accumulator's four steps, the three FMAs and the sum over the groups
+    split = np.sqrt(B) * np.linalg.norm(W, axis=0) * quantum / np.sqrt(12)
+    f32 = np.sqrt(B) * 8 * 2.0 ** -24 * 15 * big * np.linalg.norm(s.astype(np.float64), axis=0)
+    assert (err <= 1.5 * split + f32).all(), (err / (1.5 * split + f32)).max()
+
+
 def test_infinity_and_nan_show(monkeypatch):
     from gpu_util import dev_weight, randn_bf16, synth_awq, to_dev, to_host
     from mlir_air_b200 import ops
