@@ -25,9 +25,10 @@ def _nan(*shape):
 
 # unit of 32 token rows, piece of up to 256, two k-blocks of 64 at a time, 256 columns per pair (128 per CTA):
 # one row; a row either side of a unit; of the two-set limit (128); of a piece; rounds and remainders over several column
-# tiles; the second CTA's columns missing, partly missing, complete
+# tiles, meeting at the edge of one and inside one, with cuts moved to an edge, with one accumulator set and with two; the second
+# CTA's columns missing, partly missing, complete
 SHAPES = [(1, 128, 32), (31, 128, 128), (33, 256, 160), (128, 384, 256), (129, 384, 288), (256, 128, 512), (257, 640, 96),
-          (300, 256, 2400), (777, 256, 1056), (1030, 128, 4128), (96, 1024, 20480)]
+          (300, 256, 2400), (777, 256, 1056), (1030, 128, 4128), (96, 1024, 20480), (700, 256, 9600), (600, 128, 19968), (900, 384, 12992)]
 
 
 @pytest.mark.parametrize("M,K,N", SHAPES)
@@ -56,8 +57,9 @@ def test_bf16_edges(ops, M, K, N):
     assert O.rel_l2(y, ref) <= 1e-3
 
 
-# sizes whose cheapest plan is a round of whole tiles and a rest, cut evenly, that begins inside a column tile
-@pytest.mark.parametrize("M,K,N", [(160, 2048, 6400), (300, 4096, 3840), (129, 1024, 6145), (192, 512, 6272), (288, 512, 3840), (320, 512, 3600)])
+# sizes at which a plan of one round of whole tiles and a rest that begins inside a column tile, two units before its edge, would be
+# the cheapest if those two units were nobody's; and one whose rounds and rest do meet inside a column tile
+@pytest.mark.parametrize("M,K,N", [(160, 2048, 6400), (300, 4096, 3840), (129, 1024, 6145), (192, 512, 6272), (288, 512, 3840), (320, 512, 3600), (2000, 512, 9000)])
 @pytest.mark.parametrize("scratch", [True, False])
 def test_bf16_round_and_rest(ops, M, K, N, scratch):
     import torch

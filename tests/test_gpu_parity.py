@@ -407,8 +407,8 @@ def test_gemm_tensor_core_kernel(ops, M, K, N):
 @pytest.mark.parametrize("M,K,N", [(192, 128, 256), (1, 128, 32), (130, 384, 288), (300, 1024, 1056), (512, 2048, 768), (2048, 512, 256),
                                    (65, 256, 4096)])
 def test_gemm_tensor_memory_kernel(ops, M, K, N):
-    """The tcgen05 kernel that keeps the dequantised weights in tensor memory (operands swapped, 192-row tiles): ragged
-    row and column tiles, several tiles per CTA, all three epilogues, against both goldens."""
+    """The tcgen05 kernel under its other name ("tm": the same kernel as "tc"): ragged row and column tiles, one and two
+    accumulator sets, all three epilogues, against both goldens."""
     ops.set_gemm_kernel("tm")
     try:
         qw, qz, s = synth_awq(K, N, 128, seed=3 * M + N)
