@@ -75,7 +75,8 @@ constexpr int FF_MAX_LAYERS = 1024;  // 2 claim words per layer in shared memory
 // (it grows by four per layer), and per k-group of the gate/up projection (128 hidden values) how many of its two
 // 64-column sub-strips (two per layer); then one f32 sum of squares per (layer boundary, batch row).
 constexpr size_t FF_STATE_OFF = SK_WS_END;
-// Words that one SM counts up while others poll them lie in sectors of their own (side by side, 70B layer: 74.0 -> 73.1 us).
+// Words that one SM counts up while others poll them lie in sectors of their own (side by side, 70B layer in a short burst: 74.0 -> 73.1 us; in a loop of
+// seconds at the power cap no difference beyond the runs' own).
 constexpr size_t FF_STATE_HEADER = 512;
 constexpr int FF_DONE_STRIDE = 64, FF_READY_STRIDE = 8;
 constexpr int FF_READY_WORDS = 1024;  // >= SK_MAX_GROUPS, per direction

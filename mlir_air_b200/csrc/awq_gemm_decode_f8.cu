@@ -694,7 +694,8 @@ int launch_gemv_rows(const uint16_t *x, const int32_t *qweight, const int32_t *q
 // 70B layer against 129: its promote warps' chain is 1,640 cycles per unit, and one half waits for the other.)  Measured
 // in a replayed graph, us per layer at 16 / 32 rows, before (a launch of its own for every split, and the second pass adding
 // its contributors one after another) -> now: hidden 2048, intermediate 8192 26.6 / 30.1 -> 22.1 / 24.4; 4096, 11008 36.9 / 41.1 ->
-// 31.2 / 35.3; 8192, 28672 99 / 105 -> 86 / 99 (in a loop of seconds the last is held at 120 by the power cap either way).  Called
+// 31.2 / 35.3; 8192, 28672 94 / 105 -> 87 / 102 in a short burst (in a loop of seconds at the power cap 102 / 121 -> 98.5 / 121.5: the clock falls as
+// the work per cycle rises).  Called
 // without a graph the layer is one call from the host instead of five to seven: 46.9 -> 28.1 us at hidden 2048.
 bool ffn_layer_supported(int M, int H, int I, int group_size) {
     return gemm_decode_supported(M, H, 2 * I, group_size) && gemm_decode_supported(M, I, H, group_size) &&

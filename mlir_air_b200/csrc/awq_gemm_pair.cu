@@ -10,6 +10,7 @@
 // dequantised weights as a shared-memory tile / in tensor memory with 192-row tiles dealt round-robin):
 //   128 x 4096 x 14336   35 -> 20      512 x 4096 x 14336   59 -> 50     2048 x 4096 x 14336   202 -> 173 (1.39 PFLOP/s)
 //   128 x 14336 x 4096  105 -> 50      777 x 14336 x 4096  106 -> 73     4096 x 8192 x 57344  3350 -> 3090
+// These are short bursts; in a loop of seconds at the power cap 2048 x 4096 x 14336 takes 227 -> 200.
 // With scratch from the caller, K cut into parts (uncut -> cut, second pass included): 128 x 14336 x 4096 49 -> 23, 256 x 8192 x 2048
 // 31 -> 18, 65 x 4096 x 4096 19 -> 13.5; bf16 weights 512 x 8192 x 2048 34 -> 24.  Letting the next launch start early (programmatic
 // dependent launch) takes 1 to 2 us off each launch in a row: 96 x 512 x 1024 8.2 -> 6.0.
@@ -23,8 +24,8 @@
 //            range per pair, so that no pair idles in a partial last wave whatever M and N are; a range is walked in
 //            pieces of nearly equal width inside a column tile.  Where the cuts may lie is chosen on the host by a cost
 //            model (awq_pair_plan.cuh)
-//   TMEM     int4: accumulators at 0 (two sets of 192 columns, or one of 256), four weight buffers of 32 columns (64 k)
-//            from 384 on; bf16: two accumulator sets of 256
+//   TMEM     int4: accumulators at 0 (two sets of 128 columns, or one of 256), eight weight buffers of 32 columns (64 k)
+//            from 256 on; bf16: two accumulator sets of 256
 //   epilogue accumulators -> bf16 (or f32 + residual -> bf16) -> stmatrix.trans into a staging tile in shared memory ->
 //            16-byte row stores; the accumulators are free again after about a thousand cycles, the stores overlap the next piece
 //
@@ -50,6 +51,8 @@ constexpr int GP_EPI_WARPS = 8;
 constexpr int GP_STAGING_STRIDE = GP_HALF * 2 + 16;        // bytes of a token row in the staging tile (+16: no bank conflicts)
 constexpr uint32_t GP_TMEM_COLS = 512;
 constexpr int GP_ABUF = 8, GP_ABUF_COLS = GP_BK / 2, GP_ABUF_COL0 = 256;
+static_assert(2 * GP_UNIT * GP_MAX_UNITS <= (int)GP_TMEM_COLS, "two accumulator sets (bf16)");
+static_assert(GP_UNIT * GP_MAX_UNITS <= GP_ABUF_COL0 && GP_ABUF_COL0 + GP_ABUF * GP_ABUF_COLS <= (int)GP_TMEM_COLS, "accumulators, then weight buffers (int4)");
 constexpr int GP_DEQUANT_GROUPS = 4;
 constexpr int GP_MAX_STAGES = 12, GP_DONE_RING = 16;
 

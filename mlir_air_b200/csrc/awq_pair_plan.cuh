@@ -72,8 +72,10 @@ struct PairWalk {
 // The longest pair's time for a plan, in cycles.  Measured with clock64 per k-block of 64: 69 cycles per unit of 32 token
 // rows (64 at the tensor pipe's peak), but not less than about 370 with int4 weights (the chain of a dequant group: fetch
 // 240, arithmetic 630, tensor-memory store 200, over four groups) and 280 plus 35 per unit with bf16 ones (its bytes at the
-// 59 bytes per cycle and SM that L2 delivers: a narrow piece's stage is mostly weights).  A piece's drain is exposed where there is one accumulator set: 2,600 cycles.  Parts of K: their sums
-// cross L2 twice, and the second pass is a launch.
+// 59 bytes per cycle and SM that L2 delivers: a narrow piece's stage is mostly weights).  With one accumulator set a piece's drain is
+// exposed: what a second and a third piece of 256 rows add beyond their multiplications is 2,700 to 4,000 cycles (74 column tiles,
+// K 1024 and 2048), charged as 3,000.  With two sets it overlaps the next piece; the 600 charged for a piece are an estimate.
+// Parts of K: their sums cross L2 twice, and the second pass is a launch.
 inline size_t pair_parts_bytes(int M, int N, int S) { return (size_t)S * M * ((N + GP_BN - 1) / GP_BN * GP_BN) * 4; }
 constexpr size_t GP_PARTS_MAX_BYTES = 64u << 20;  // about half of L2
 inline long long pair_cost(const PairPlan &pl, int KB_all, bool w4, int M) {
