@@ -229,6 +229,8 @@ class DecodeFFNStack:
             return False
         return all(self.gemm_ws.fits_f8(batch, w.K, w.N) for l in self.layers for w in (l.gateup, l.down))
 
+    one_call = True  # (the constructor's argument; a default for the accounting of a stack made without it)
+
     def uses_layer(self, batch: int) -> bool:
         """One GPU: each layer is one call (fp8-operand kernel up to 32 rows, 16-bit one beyond)."""
         if self.tp > 1 or not self.one_call or self.GEMM_F8_MIN_WEIGHTS != DecodeFFNStack.GEMM_F8_MIN_WEIGHTS or not self.uses_gemm(batch):
