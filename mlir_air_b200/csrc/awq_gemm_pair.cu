@@ -50,11 +50,9 @@ constexpr int GP_X_UNIT_BYTES = GP_UNIT / 2 * GP_BK * 2;   // 2 KB: this CTA's h
 constexpr int GP_EPI_WARPS = 8;
 constexpr int GP_STAGING_STRIDE = GP_HALF * 2 + 16;        // bytes of a token row in the staging tile (+16: no bank conflicts)
 constexpr uint32_t GP_TMEM_COLS = 512;
-constexpr int GP_ABUF = 8, GP_ABUF_COLS = GP_BK / 2, GP_ABUF_COL0 = 256;
+constexpr int GP_ABUF_COLS = GP_BK / 2, GP_ABUF_COL0 = 256;
 static_assert(2 * GP_UNIT * GP_MAX_UNITS <= (int)GP_TMEM_COLS, "two accumulator sets (bf16)");
 static_assert(GP_UNIT * GP_MAX_UNITS <= GP_ABUF_COL0 && GP_ABUF_COL0 + GP_ABUF * GP_ABUF_COLS <= (int)GP_TMEM_COLS, "accumulators, then weight buffers (int4)");
-constexpr int GP_DEQUANT_GROUPS = 4;
-constexpr int GP_MAX_STAGES = 12, GP_DONE_RING = 16;
 
 template <bool W4>
 struct PairCfg {
@@ -62,11 +60,11 @@ struct PairCfg {
     static constexpr int S_BYTES = W4 ? GP_HALF * 2 : 0, Z_BYTES = W4 ? GP_HALF / 8 * 4 : 0;
     // Warps that load, on alternate k-blocks: a k-block costs a loading warp about 430 cycles (a look at a barrier 120, four
     // copies 180, the rest the loop), which one warp alone turned into the launch's time for pieces narrower than 200 rows.
-    static constexpr int PRODUCERS = W4 ? 3 : 2;
+    static constexpr int PRODUCERS = W4 ? GP_PRODUCERS_INT4 : GP_PRODUCERS_BF16;
     static constexpr int DEQUANT_WARPS = W4 ? 4 * GP_DEQUANT_GROUPS : 0;
     static constexpr int EPI_WARP0 = 4 + DEQUANT_WARPS;
     static constexpr int THREADS = (EPI_WARP0 + GP_EPI_WARPS) * 32;
-    static constexpr int NUM_BARS = GP_MAX_STAGES + GP_ABUF / 2 + GP_DONE_RING + 4;
+    static constexpr int NUM_BARS = 2 * GP_BAR_RING + GP_ABUF / 2 + 4;
     static constexpr int BAR_BYTES = (NUM_BARS * 8 + 16 + 127) / 128 * 128;
     // token rows that go through the staging tile at a time: all of a piece (int4: the accumulators must be free again
     // quickly, there may be one set only), or 64 (bf16: two sets, the room goes to stages)
@@ -212,14 +210,14 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, uint16_t *__restrict__ C
     const uint32_t bar_base = smem_base + (uint32_t)(stages * lay.stage_bytes);
     const uint32_t staging = bar_base + Cfg::BAR_BYTES;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_gen + stages * lay.stage_bytes + Cfg::NUM_BARS * 8);
-    // int4: TMA landed in stage s of this CTA; bf16: in stage s of both CTAs (leader's)
-    auto full_bar = [&](int s) { return bar_base + 8u * s; };
+    // k-block i has landed: int4 in this CTA; bf16 in both (leader's)
+    auto full_bar = [&](int i) { return bar_base + 8u * pair_bar(i); };
     // int4, leader's: weight buffers 2 b and 2 b + 1 are dequantised in both CTAs
-    auto ready_bar = [&](int b) { return bar_base + 8u * (GP_MAX_STAGES + b); };
-    // the pair's MMAs of k-block i are done, barrier i % 16: frees its stage and its weight buffer
-    auto done_bar = [&](int i) { return bar_base + 8u * (GP_MAX_STAGES + GP_ABUF / 2 + (i & (GP_DONE_RING - 1))); };
-    auto acc_full = [&](int a) { return bar_base + 8u * (GP_MAX_STAGES + GP_ABUF / 2 + GP_DONE_RING + a); };
-    auto acc_empty = [&](int a) { return bar_base + 8u * (GP_MAX_STAGES + GP_ABUF / 2 + GP_DONE_RING + 2 + a); };  // (leader's)
+    auto ready_bar = [&](int b) { return bar_base + 8u * (GP_BAR_RING + b); };
+    // the pair's MMAs of k-block i are done: frees its stage and its weight buffer
+    auto done_bar = [&](int i) { return bar_base + 8u * (GP_BAR_RING + GP_ABUF / 2 + pair_bar(i)); };
+    auto acc_full = [&](int a) { return bar_base + 8u * (2 * GP_BAR_RING + GP_ABUF / 2 + a); };
+    auto acc_empty = [&](int a) { return bar_base + 8u * (2 * GP_BAR_RING + GP_ABUF / 2 + 2 + a); };  // (leader's)
     auto stage_addr = [&](int s) { return smem_base + (uint32_t)(s * lay.stage_bytes); };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -231,9 +229,11 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, uint16_t *__restrict__ C
     PairWalk walk(pair - part * plan.P, plan);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < stages; ++s) mbar_init(full_bar(s), 1);
         for (int b = 0; b < GP_ABUF / 2; ++b) mbar_init(ready_bar(b), 16);  // per k-block four dequant warps in each CTA
-        for (int i = 0; i < GP_DONE_RING; ++i) mbar_init(done_bar(i), 1);
+        for (int i = 0; i < GP_BAR_RING; ++i) {
+            mbar_init(full_bar(i), 1);
+            mbar_init(done_bar(i), 1);
+        }
         for (int a = 0; a < 2; ++a) {
             mbar_init(acc_full(a), 1);
             mbar_init(acc_empty(a), 2 * GP_EPI_WARPS);
@@ -272,12 +272,12 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, uint16_t *__restrict__ C
             const uint32_t tx = (uint32_t)half_rows * GP_BK * 2 + Cfg::W_BYTES + Cfg::S_BYTES + Cfg::Z_BYTES;
             for (; kb < KB; kb += Cfg::PRODUCERS, it += Cfg::PRODUCERS) {
                 const int freed = it - stages;  // the k-block that had the stage before
-                if (freed >= 0 && !mbar_wait_bounded_warp(done_bar(freed), (freed / GP_DONE_RING) & 1, wait_limit)) {
+                if (freed >= 0 && !mbar_wait_bounded_warp(done_bar(freed), pair_bar_parity(freed), wait_limit)) {
                     if (lane == 0) atomicExch(&g_gemm_pair_error, 1);
                     ok = false;
                     break;
                 }
-                const uint32_t st = stage_addr(s), bar = full0 + 8u * s;
+                const uint32_t st = stage_addr(s), bar = full0 + 8u * pair_bar(it);
                 const int k0 = (kb_first + kb) * GP_BK;
                 if (elect_one()) {
                     if (W4) {
@@ -288,7 +288,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, uint16_t *__restrict__ C
                         tma_load_2d(st + x_bytes + Cfg::W_BYTES + Cfg::S_BYTES, &maps.z, n0 / 8, g, bar);
                         tma_load_2d(st, mx, k0, m0, bar);
                     } else {
-                        if (rank == 0) mbar_expect_tx(full_bar(s), 2 * tx);  // both CTAs' copies are counted on the leader's barrier
+                        if (rank == 0) mbar_expect_tx(full_bar(it), 2 * tx);  // both CTAs' copies are counted on the leader's barrier
                         gp_tma_load_2d_pair(st, mx, k0, m0, bar);
                         gp_tma_load_2d_pair(st + x_bytes, &maps.w, k0, n0, bar);
                     }
@@ -301,10 +301,10 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, uint16_t *__restrict__ C
     } else if (warp == 1) {
         // ------------------------------ MMA issuer (leader CTA only) ------------------------------
         if (rank == 0) {
-            // What is looked at: int4 the four barriers of the weight buffer pairs, bf16 the stages.  Two k-blocks take eight
+            // What is looked at: int4 the four barriers of the weight buffer pairs, bf16 those of the k-blocks.  Two k-blocks take eight
             // MMAs, two commits and one look at most: a k-block at a time, the issuing warp's own instructions (a look costs
             // a hundred cycles even when it is over at once) took 430 cycles per k-block however narrow the piece.
-            const int ring = W4 ? GP_ABUF / 2 : stages;
+            constexpr int ring = W4 ? GP_ABUF / 2 : GP_BAR_RING, look = W4 ? ring : 8;  // (every lane that looks costs: 16 of them 2 %)
             constexpr int STEP = W4 ? 1 : 2;  // barriers per two k-blocks
             int s = 0, r = 0, rphase = 0, piece = 0, avail = 0, j = 0;
             bool ok = true;
@@ -321,7 +321,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, uint16_t *__restrict__ C
                     if (avail < STEP) {
                         const int b = r + lane < ring ? r + lane : r + lane - ring;
                         const uint32_t parity = r + lane < ring ? rphase : rphase ^ 1;
-                        avail = gp_count_ready<STEP>(lane < ring ? (W4 ? ready_bar(b) : full_bar(b)) : 0u, parity, wait_limit);
+                        avail = gp_count_ready<STEP>(lane < look ? (W4 ? ready_bar(b) : full_bar(b)) : 0u, parity, wait_limit);
                         if (avail == 0) {
                             if (lane == 0) atomicExch(&g_gemm_pair_error, 3);
                             ok = false;
@@ -371,10 +371,10 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, uint16_t *__restrict__ C
         const uint32_t ready0 = gp_mapa(ready_bar(0), 0);
         int units = 0;
         while (walk.next()) units += KB;
-        int s = grp, phase = 0;
+        int s = grp;
         for (int it = grp; it < units; it += GP_DEQUANT_GROUPS) {
             const int ab = it % GP_ABUF, freed = it - GP_ABUF;  // the k-block that had the buffer before
-            if (!mbar_wait_bounded(full_bar(s), phase, wait_limit)) {
+            if (!mbar_wait_bounded(full_bar(it), pair_bar_parity(it), wait_limit)) {
                 if (lane == 0) atomicExch(&g_gemm_pair_error, 4);
                 break;
             }
@@ -404,7 +404,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, uint16_t *__restrict__ C
                     d[4 * c + 2 * (e & 1) + 1] = v1;
                 }
             }
-            if (freed >= 0 && !mbar_wait_bounded(done_bar(freed), (freed / GP_DONE_RING) & 1, wait_limit)) {
+            if (freed >= 0 && !mbar_wait_bounded(done_bar(freed), pair_bar_parity(freed), wait_limit)) {
                 if (lane == 0) atomicExch(&g_gemm_pair_error, 4);
                 break;
             }
@@ -417,7 +417,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, uint16_t *__restrict__ C
             __syncwarp();
             if (lane == 0) gp_arrive_cluster(ready0 + 8u * (ab >> 1));
             s += GP_DEQUANT_GROUPS;
-            if (s >= stages) s -= stages, phase ^= 1;
+            if (s >= stages) s -= stages;
         }
     } else if (warp >= Cfg::EPI_WARP0) {
         // ------------------------------ epilogue ------------------------------

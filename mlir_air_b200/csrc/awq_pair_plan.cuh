@@ -17,6 +17,18 @@ constexpr int GP_BN = 256, GP_BK = 64;         // weight columns of a pair, k of
 constexpr int GP_UNIT = 32, GP_MAX_UNITS = 8;  // token rows: unit of the schedule, most units per piece
 constexpr int GP_MAX_PARTS = 8;                // parts of K
 
+// Hand-over of k-blocks, counted through all pieces of a launch: k-block i lies in stage i % stages, is dequantised (int4) by warp group
+// i % 4 into weight buffer i % 8, and has two barriers, "landed" and "multiplied", each in a ring of 16 by its own number.
+// A wait for a phase by its parity takes the phase before the last for the one it means, so whoever waits for k-block i must
+// know that k-block i - 16's phase of the same barrier is over.  It does: a warp that is at i has waited for "multiplied" of
+// i - 12 (a dequant warp, at its step before), which is after "landed" of it, or of i - 3 - stages (a producer; 12 stages at
+// most).  The stage's own number would not do for "landed": with 7 stages, k-block i - 7 is another group's, and may still be on
+// its way while group i % 4 looks for i; its wait returned at once then, and it dequantised what the stage held before.
+constexpr int GP_BAR_RING = 16;
+GP_HD inline int pair_bar(int i) { return i & (GP_BAR_RING - 1); }
+GP_HD inline int pair_bar_parity(int i) { return (i / GP_BAR_RING) & 1; }
+constexpr int GP_MAX_STAGES = 12, GP_ABUF = 8, GP_DEQUANT_GROUPS = 4, GP_PRODUCERS_INT4 = 3, GP_PRODUCERS_BF16 = 2;
+
 // The schedule of a launch.  Token rows are counted in units of 32, R of them per column tile.  First `waves` rounds in
 // which the P pairs take neighbouring tiles of the (column tile, token tile) grid, token tiles innermost (N_T nearly equal
 // ones per column tile): the pairs of a round share token rows and weights in L2.  What does not fill a round is cut

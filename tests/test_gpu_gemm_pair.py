@@ -104,6 +104,23 @@ def test_runs_back_to_back_are_independent(ops):
     assert torch.equal(chained, synced)
 
 
+@pytest.mark.parametrize("M,K,N", [(3000, 4096, 2048), (4096, 8192, 1056), (2048, 2048, 4096)])
+def test_int4_deep_products_repeat(ops, M, K, N):
+    """Pieces of 256 token rows, whose ring has seven stages, and token rows that come from HBM: k-blocks land out of order and the
+    dequant groups look for them at very different times.  Each run gives the same bits."""
+    import torch
+    w, A = dev_weight(*synth_awq(K, N, 128, seed=5)), torch.randn((M, K), device="cuda").to(torch.bfloat16)
+    flush = torch.empty(1 << 28, dtype=torch.uint8, device="cuda")  # twice the L2
+    first = ops.gemm(A, w)
+    ref = A.double() @ ops.dequant(w).double()
+    assert ((first.double() - ref).norm() <= 3e-3 * ref.norm()).item()  # one bf16 rounding; a k-block of K / 64 that is wrong is 0.1 in its piece
+    for i in range(60):
+        if i % 2:
+            flush.fill_(i)
+        assert torch.equal(ops.gemm(A, w, out=_nan(M, N)), first), i
+    ops.gemm_check()
+
+
 # K cut into parts: one piece per part, ragged last tiles and rows, parts of unequal length, N that takes scalar stores
 @pytest.mark.parametrize("M,K,N", [(65, 4096, 4096), (16, 8192, 256), (100, 2048, 544), (300, 8192, 2048), (257, 14336, 1056), (40, 1152, 32)])
 def test_int4_k_parts(ops, M, K, N):

@@ -88,3 +88,96 @@ def test_plans_cover_every_unit_once(checker, kind):
     outs = [p.communicate()[0] for p in procs]
     assert all(p.returncode == 0 for p in procs), "".join(o for o, p in zip(outs, procs) if p.returncode)
     assert sum(int(o.split()[0]) for o in outs) > 100000
+
+
+# The hand-over of k-blocks between the int4 kernel's warp roles, step by step with random durations: barriers are counters of finished
+# phases that a waiter sees only as a parity, as mbarrier.test_wait shows them.  Each wait that returns is compared with what
+# has really happened.
+HANDOVER = r"""
+#include <cstdio>
+#include <cstdlib>
+#include <random>
+#include <vector>
+#include "awq_pair_plan.cuh"
+using namespace awq;
+
+static std::mt19937 rng;
+static int upto(int n) { return (int)(rng() % (unsigned)n); }
+struct Bars {
+    std::vector<int> phases = std::vector<int>(64, 0);
+    bool looks_over(int b, int parity) const { return (phases[b] & 1) != parity; }
+};
+struct Role {
+    int i, step, state = 0, until = 0;
+};
+// `by_stage`: "landed" barriers numbered by the stage
+static int run(int stages, int n, int slow, bool by_stage) {
+    Bars landed, multiplied;
+    std::vector<int> load_end(n, -1), has_landed(n, 0), has_multiplied(n, 0), ready(n, 0);
+    auto lb = [&](int i) { return by_stage ? i % stages : pair_bar(i); };
+    auto lp = [&](int i) { return by_stage ? i / stages & 1 : pair_bar_parity(i); };
+    std::vector<Role> producers, groups;
+    for (int p = 0; p < GP_PRODUCERS_INT4; ++p) producers.push_back({p, GP_PRODUCERS_INT4});
+    for (int g = 0; g < GP_DEQUANT_GROUPS; ++g) groups.push_back({g, GP_DEQUANT_GROUPS});
+    int mma = 0, mma_until = 0;
+    for (int t = 0; has_multiplied[n - 1] == 0; ++t) {
+        if (t > 4000 * n) return 2;  // nobody moves any more
+        for (int i = 0; i < n; ++i)
+            if (load_end[i] == t) has_landed[i] = 1, ++landed.phases[lb(i)];
+        for (Role &p : producers) {
+            if (p.i >= n) continue;
+            const int freed = p.i - stages;
+            if (freed >= 0) {
+                if (!multiplied.looks_over(pair_bar(freed), pair_bar_parity(freed))) continue;
+                if (!has_multiplied[freed]) return 1;
+            }
+            load_end[p.i] = t + 5 + upto(20) + (upto(8) == 0 ? upto(slow) : 0);
+            p.i += p.step;
+        }
+        for (Role &g : groups) {
+            if (g.i >= n || t < g.until) continue;
+            if (g.state == 0) {  // looks for its k-block, reads and converts it
+                if (!landed.looks_over(lb(g.i), lp(g.i))) continue;
+                if (!has_landed[g.i]) return 1;
+                g.state = 1, g.until = t + 4 + upto(8);
+            } else if (g.state == 1) {  // looks for its weight buffer, writes it
+                const int freed = g.i - GP_ABUF;
+                if (freed >= 0) {
+                    if (!multiplied.looks_over(pair_bar(freed), pair_bar_parity(freed))) continue;
+                    if (!has_multiplied[freed]) return 1;
+                }
+                g.state = 2, g.until = t + 1 + upto(3);
+            } else {
+                ready[g.i] = 1;
+                g.i += g.step, g.state = 0;
+            }
+        }
+        if (t >= mma_until && ready[mma] && ready[mma + 1]) {
+            for (int k = 0; k < 2; ++k) has_multiplied[mma + k] = 1, ++multiplied.phases[pair_bar(mma + k)];
+            mma += 2, mma_until = t + 2 + upto(6);
+            if (mma >= n) break;
+        }
+    }
+    return 0;
+}
+int main(int, char **argv) {
+    const bool by_stage = std::atoi(argv[1]) != 0;
+    int early = 0, stuck = 0;
+    for (int stages = 6; stages <= GP_MAX_STAGES; ++stages)
+        for (int seed = 0; seed < 400; ++seed) {
+            rng.seed(1000 * stages + seed);
+            const int r = run(stages, 64, 10 << seed % 6, by_stage);
+            early += r == 1, stuck += r == 2;
+        }
+    std::printf("%d %d\n", early, stuck);
+}
+"""
+
+
+def test_no_wait_for_a_k_block_returns_early(tmp_path):
+    src, exe = tmp_path / "handover.cpp", tmp_path / "handover"
+    src.write_text(HANDOVER)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-Wall", "-I", CSRC, str(src), "-o", str(exe)], check=True)
+    run = lambda arg: subprocess.run([str(exe), arg], check=True, stdout=subprocess.PIPE, text=True).stdout.split()
+    assert run("0") == ["0", "0"]
+    assert int(run("1")[0]) > 0  # the model sees what barriers numbered by the stage would allow
