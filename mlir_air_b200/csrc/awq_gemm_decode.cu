@@ -85,6 +85,8 @@ struct DgCfg {
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
     static_assert(STAGE_BYTES % 1024 == 0, "swizzled tiles need 1024-byte alignment");
     static_assert(STAGES >= 3, "input ring too shallow");
+    // the k-blocks of a stage are all the same dequant group's: its wait for one, by parity, could not tell the phase before the last
+    static_assert(STAGES % 2 == 0, "two dequant groups on alternate units");
 };
 
 __device__ int g_gemm_dec_error;  // 0 = ok; set when a bounded wait gave up
