@@ -45,10 +45,7 @@ namespace awq {
 int encode_tensor_map_2d(CUtensorMap *map, int dtype, const void *base, uint64_t dim0, uint64_t dim1,
                          uint64_t stride1_bytes, uint32_t box0, uint32_t box1, int swizzle);
 
-constexpr int GP_HALF = 128, GP_GROUP = 128;
-constexpr int GP_X_UNIT_BYTES = GP_UNIT / 2 * GP_BK * 2;   // 2 KB: this CTA's half of a unit of token rows x 64 k
 constexpr int GP_EPI_WARPS = 8;
-constexpr int GP_STAGING_STRIDE = GP_HALF * 2 + 16;        // bytes of a token row in the staging tile (+16: no bank conflicts)
 constexpr uint32_t GP_TMEM_COLS = 512;
 constexpr int GP_ABUF_COLS = GP_BK / 2, GP_ABUF_COL0 = 256;
 static_assert(2 * GP_UNIT * GP_MAX_UNITS <= (int)GP_TMEM_COLS, "two accumulator sets (bf16)");
@@ -56,35 +53,14 @@ static_assert(GP_UNIT * GP_MAX_UNITS <= GP_ABUF_COL0 && GP_ABUF_COL0 + GP_ABUF *
 
 template <bool W4>
 struct PairCfg {
-    static constexpr int W_BYTES = W4 ? GP_BK * (GP_HALF / 8) * 4 : GP_HALF * GP_BK * 2;  // 4 KB of packed words / 16 KB of bf16
-    static constexpr int S_BYTES = W4 ? GP_HALF * 2 : 0, Z_BYTES = W4 ? GP_HALF / 8 * 4 : 0;
+    static constexpr int W_BYTES = pair_w_bytes(W4), S_BYTES = pair_s_bytes(W4), Z_BYTES = pair_z_bytes(W4);
     // Warps that load, on alternate k-blocks: a k-block costs a loading warp about 430 cycles (a look at a barrier 120, four
     // copies 180, the rest the loop), which one warp alone turned into the launch's time for pieces narrower than 200 rows.
     static constexpr int PRODUCERS = W4 ? GP_PRODUCERS_INT4 : GP_PRODUCERS_BF16;
     static constexpr int DEQUANT_WARPS = W4 ? 4 * GP_DEQUANT_GROUPS : 0;
     static constexpr int EPI_WARP0 = 4 + DEQUANT_WARPS;
     static constexpr int THREADS = (EPI_WARP0 + GP_EPI_WARPS) * 32;
-    static constexpr int NUM_BARS = 2 * GP_BAR_RING + GP_ABUF / 2 + 4;
-    static constexpr int BAR_BYTES = (NUM_BARS * 8 + 16 + 127) / 128 * 128;
-    // token rows that go through the staging tile at a time: all of a piece (int4: the accumulators must be free again
-    // quickly, there may be one set only), or 64 (bf16: two sets, the room goes to stages)
-    static constexpr int STAGING_UNITS = W4 ? GP_MAX_UNITS : 2;
 };
-constexpr int GP_SMEM_MAX = 227 * 1024;
-// What a launch makes of its shared memory; widths are those of its widest piece.
-struct PairLayout {
-    int stage_bytes, stages, staging_rows;
-};
-template <bool W4>
-__host__ __device__ inline PairLayout pair_layout(int max_units) {
-    using Cfg = PairCfg<W4>;
-    PairLayout l;
-    l.stage_bytes = (max_units * GP_X_UNIT_BYTES + Cfg::W_BYTES + Cfg::S_BYTES + Cfg::Z_BYTES + 1023) / 1024 * 1024;
-    l.staging_rows = GP_UNIT * (max_units < Cfg::STAGING_UNITS ? max_units : Cfg::STAGING_UNITS);
-    const int room = GP_SMEM_MAX - 1024 - Cfg::BAR_BYTES - l.staging_rows * GP_STAGING_STRIDE;
-    l.stages = room / l.stage_bytes < GP_MAX_STAGES ? room / l.stage_bytes : GP_MAX_STAGES;
-    return l;
-}
 // f32 accumulate, bf16 x bf16, both K-major, M 256 over the pair; N is added per piece
 constexpr uint32_t GP_IDESC_BASE = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 4) << 24);
 
@@ -204,12 +180,12 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, uint16_t *__restrict__ C
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-    const PairLayout lay = pair_layout<W4>(plan.max_units);
+    const PairLayout lay = pair_layout(W4, plan.max_units);
     const int stages = lay.stages, acc_sets = plan.sets;
     const int x_bytes = plan.max_units * GP_X_UNIT_BYTES;
     const uint32_t bar_base = smem_base + (uint32_t)(stages * lay.stage_bytes);
-    const uint32_t staging = bar_base + Cfg::BAR_BYTES;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_gen + stages * lay.stage_bytes + Cfg::NUM_BARS * 8);
+    const uint32_t staging = bar_base + GP_BAR_BYTES;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_gen + stages * lay.stage_bytes + GP_NUM_BARS * 8);
     // k-block i has landed: int4 in this CTA; bf16 in both (leader's)
     auto full_bar = [&](int i) { return bar_base + 8u * pair_bar(i); };
     // int4, leader's: weight buffers 2 b and 2 b + 1 are dequantised in both CTAs
@@ -664,8 +640,8 @@ static int launch_pair(const uint16_t *A, const void *w, const int32_t *qzeros, 
     if (attr_err != cudaSuccess) return check_cuda(attr_err, "pair gemm: shared memory attribute");
     PairPlan plan = pair_plan<W4>(M, N, K, pair_count(), workspace != nullptr);
     if (plan.S > 1 && workspace_bytes < pair_parts_bytes(M, N, plan.S)) plan = pair_plan<W4>(M, N, K, pair_count(), false);
-    const PairLayout lay = pair_layout<W4>(plan.max_units);
-    const size_t smem = 1024 + (size_t)lay.stages * lay.stage_bytes + Cfg::BAR_BYTES + (size_t)lay.staging_rows * GP_STAGING_STRIDE;
+    const PairLayout lay = pair_layout(W4, plan.max_units);
+    const size_t smem = 1024 + (size_t)lay.stages * lay.stage_bytes + GP_BAR_BYTES + (size_t)lay.staging_rows * GP_STAGING_STRIDE;
     PairMaps maps;
     int rc;
     for (int u = 1; u <= plan.max_units; ++u)

@@ -66,7 +66,11 @@ int main(int argc, char **argv) {
     for (int C = C_first; C <= 120; C += 3 * C_step)
         for (int R = 1; R <= 70; R += R < 24 ? 1 : 5)
             for (int pairs = 60; pairs <= 80; pairs += 1 + C % 3)
-                pair_candidates(32 * R, 256 * C, 8192, pairs, w4, true, [&](const PairPlan &pl) { check(w4, 32 * R, 256 * C, 8192, pairs, true, pl, "considered"); });
+            {
+                auto consider = [&](const PairPlan &pl) { check(w4, 32 * R, 256 * C, 8192, pairs, true, pl, "considered"); };
+                pair_candidates(32 * R, 256 * C, 8192, pairs, w4, true, consider);
+                if (w4) pair_even_candidates(32 * R, 256 * C, pairs, consider);
+            }
     std::printf("%lld plans\n", n_plans);
 }
 """
