@@ -114,9 +114,10 @@ struct PairWalk {
 // `ring`: with what the number of stages does to int4 pieces (pair_search says where).  A k-block takes about 4,500 cycles from the
 // request of its stage to the end of its MMAs, so no piece takes less than that over the number of stages, which its width
 // leaves room for: 7 with eight units, 10 with six, 12 with up to five.
+// `limit`: from this figure on (0: nowhere) it need not be exact.
 inline size_t pair_parts_bytes(int M, int N, int S) { return (size_t)S * M * ((N + GP_BN - 1) / GP_BN * GP_BN) * 4; }
 constexpr size_t GP_PARTS_MAX_BYTES = 64u << 20;  // about half of L2
-inline long long pair_cost(const PairPlan &pl, int KB_all, bool w4, int M, bool ring = false) {
+inline long long pair_cost(const PairPlan &pl, int KB_all, bool w4, int M, bool ring = false, long long limit = 0) {
     const int KB = (KB_all / 2 + pl.S - 1) / pl.S * 2;
     const int turn = ring ? 4500 / pair_layout(w4, pl.max_units).stages : 0;
     const int floor_cycles = ring ? (turn > 420 ? turn : 420) : (w4 ? 370 : 280), floor_unit = w4 ? 0 : 35;
@@ -136,6 +137,7 @@ inline long long pair_cost(const PairPlan &pl, int KB_all, bool w4, int M, bool 
         const int b = pl.cut(p + 1), ta = a / pl.R, tb = b / pl.R;
         const long long t = ta == tb ? cut_up(b - a) : cut_up((ta + 1) * pl.R - a) + (tb - ta - 1) * whole + cut_up(b - tb * pl.R);
         if (t > worst) worst = t;
+        if (limit && worst + rounds >= limit) break;
         a = b;
     }
     return worst + rounds;
@@ -229,13 +231,13 @@ inline PairPlan pair_search(bool w4, int M, int N, int K, int all_pairs, bool ma
     PairPlan best_plan;
     long long best = -1;
     pair_candidates(M, N, K, all_pairs, w4, may_split, [&](const PairPlan &pl) {
-        const long long c = pair_cost(pl, KB, w4, M);
+        const long long c = pair_cost(pl, KB, w4, M, false, best > 0 ? best : 0);
         if (best < 0 || c < best) best = c, best_plan = pl;
     });
     if (!w4 || best_plan.S > 1 || best_plan.waves > 0) return best_plan;
     best = pair_cost(best_plan, KB, w4, M, true);
     pair_even_candidates(M, N, all_pairs, [&](const PairPlan &pl) {
-        const long long c = pair_cost(pl, KB, w4, M, true);
+        const long long c = pair_cost(pl, KB, w4, M, true, best);
         if (c < best) best = c, best_plan = pl;
     });
     return best_plan;
