@@ -668,7 +668,7 @@ ffn_fused_kernel(const __grid_constant__ CUtensorMap tmXi, const __grid_constant
             }
             xr_parity ^= 1u << slot;
         }
-        sk_consume_unit<true>(smem_base + slot * SK_STAGE_BYTES, geo, res, empty_bar(slot), lane);
+        sk_consume_unit<true>(smem_base + slot * SK_STAGE_BYTES, geo, res, empty_bar(slot), lane, sk_opaque_zero(a.wait_limit));
     }
 }
 

@@ -175,7 +175,7 @@ gemv_streamk_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
             if (lane == 0) atomicExch(err_flag, 2);
         }
         if (!failed) {
-            sk_consume_unit<XH>(smem_base + slot * SK_STAGE_BYTES, lane_geo, res, empty_bar(slot), lane);
+            sk_consume_unit<XH>(smem_base + slot * SK_STAGE_BYTES, lane_geo, res, empty_bar(slot), lane, sk_opaque_zero(wait_limit));
         }
         if (++g == G) { g = 0; ++v; }
         if (++slot == SK_STAGES) { slot = 0; ++round; }

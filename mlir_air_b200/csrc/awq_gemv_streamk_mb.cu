@@ -209,6 +209,7 @@ gemv_streamk_mb_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
             const uint32_t st = smem_base + slot * Cfg::STAGE_BYTES;
             float acc[T][4][4];
             float sx[T][4];
+            uint32_t seen = 0;  // (sk_release_stage)
 #pragma unroll
             for (int t = 0; t < T; ++t) {
 #pragma unroll
@@ -238,6 +239,7 @@ gemv_streamk_mb_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
 #pragma unroll
                     for (int t = 0; t < T; ++t) {  // the decoded fragments serve every tile
                         const uint32_t b0 = bx[t][2 * h], b1 = bx[t][2 * h + 1];
+                        if (p == 3) seen |= R[0] | b0;
                         mma_16816<true>(sx[t], ONES, ONES, ONES, ONES, b0, b1);
 #pragma unroll
                         for (int e = 0; e < 4; ++e) mma_16816<true>(acc[t][e], a_lo[e], b_lo[e], a_hi[e], b_hi[e], b0, b1);
@@ -251,9 +253,9 @@ gemv_streamk_mb_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
             for (int e = 0; e < 4; ++e) {
                 sA[e] = lds_u16(st + s_off + 4 * e);
                 sB[e] = lds_u16(st + s_off + 64 + 4 * e);
+                seen |= sA[e] | sB[e];
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(empty_bar(slot));  // all of this warp's reads of the slot are done
+            sk_release_stage(empty_bar(slot), seen | zA | zB, sk_opaque_zero(wait_limit), lane);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 float cA = __uint_as_float(((zA << (16 - 4 * e)) & 0x000F0000u) | 0x43000000u);

@@ -275,16 +275,38 @@ struct SkLane {
     }
 };
 
+// Releasing a stage.  The arrival stands behind the reads of the stage in the source, but that alone did not make the last of them
+// (the scales, which the fix-up behind it used one by one) come first: in launches whose code and operands were not in the caches a
+// warp sometimes took the next unit's scales for its last columns (8192 x 28672 up to 1.5 % of such launches, 155 of 60,000 over
+// all sizes tried; none of 60,000 since).  So the arrival's address depends on what was read: `seen` is anything made of it,
+// `zero` a 0 that the compiler cannot know.  Waiting for the reads there costs 2 to 3 % where they stand behind the products, and
+// 0.3 % (8 rows of a 70B layer 80.2 -> 81.1 us) where they stand before them, as below.
+__device__ __forceinline__ void sk_release_stage(uint32_t empty_bar, uint32_t seen, uint32_t zero, int lane) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty_bar + (seen & zero));
+}
+// (wait limits are positive: 0)
+__device__ __forceinline__ uint32_t sk_opaque_zero(long long wait_limit) { return (uint32_t)((unsigned long long)wait_limit >> 63); }
+
 // One unit (512 columns x one group of 128 k) from the stage at shared address `st`: adds this
 // warp's 64 columns x 8 batch rows into res and releases the stage through `empty_bar`.
 template <bool XH>
 __device__ __forceinline__ void sk_consume_unit(uint32_t st, const SkLane &L, float (&res)[4][4], uint32_t empty_bar,
-                                                int lane) {
+                                                int lane, uint32_t zero) {
     const int lm = L.lm, lr = L.lr;
     const uint32_t w_off = L.w_off, z_off = L.z_off, s_off = L.s_off;
     const uint32_t ONES = XH ? 0x3C003C00u : 0x3F803F80u;
     float acc[4][4];
     float sx[4] = {0.f, 0.f, 0.f, 0.f};
+    uint32_t seen = 0;  // (sk_release_stage)
+    const uint32_t zA = lds_u16(st + z_off), zB = lds_u16(st + z_off + 16);
+    uint32_t sA[4], sB[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        sA[e] = lds_u16(st + s_off + 4 * e);
+        sB[e] = lds_u16(st + s_off + 64 + 4 * e);
+        seen |= sA[e] | sB[e];
+    }
 #pragma unroll
     for (int e = 0; e < 4; ++e)
 #pragma unroll
@@ -301,6 +323,7 @@ __device__ __forceinline__ void sk_consume_unit(uint32_t st, const SkLane &L, fl
             uint32_t R[4];  // chunk A rows 0-7, chunk A rows 8-15, chunk B rows 0-7, chunk B rows 8-15
             ldmatrix_x4_trans(R, st + (2 * p + h) * 2048 + w_off);
             const uint32_t b0 = bx[2 * h], b1 = bx[2 * h + 1];
+            if (p == 3) seen |= R[0] | b0;
             mma_16816<XH>(sx, ONES, ONES, ONES, ONES, b0, b1);
             uint32_t a_lo[4], a_hi[4], b_lo[4], b_hi[4];
             decode4<XH>(R[0], a_lo);
@@ -312,17 +335,9 @@ __device__ __forceinline__ void sk_consume_unit(uint32_t st, const SkLane &L, fl
         }
     }
 
+    sk_release_stage(empty_bar, seen | zA | zB, zero, lane);
     // group fix-up: res += s * (acc - c * sum_x); the zero point (and, for fp16, the decode
     // offset and the factor 16 of odd nibbles) live in c and s
-    const uint32_t zA = lds_u16(st + z_off), zB = lds_u16(st + z_off + 16);
-    uint32_t sA[4], sB[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        sA[e] = lds_u16(st + s_off + 4 * e);
-        sB[e] = lds_u16(st + s_off + 64 + 4 * e);
-    }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(empty_bar);  // all of this warp's reads of the slot are done
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         // 128 + z as f32: bits 0x43000000 | z << 16
