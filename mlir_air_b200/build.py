@@ -16,7 +16,8 @@ LIB_PATH = os.path.join(LIB_DIR, "libawq_b200.so")
 SOURCES = ["awq_capi.cu", "awq_dequant.cu", "awq_generic.cu", "awq_gemv_streamk.cu", "awq_gemv_streamk_mb.cu", "awq_gemm_decode.cu", "awq_gemm_decode_f8.cu", "awq_gemm_pair.cu",
            "awq_static_scratch.cu", "awq_ffn_fused.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
-              "-Xcompiler", "-Wall"]
+              "-Xcompiler", "-Wall",
+              "-Werror", "cross-execution-space-call"]  # (host code called on the device compiles, and computes nothing there)
 
 
 def _nvcc():
